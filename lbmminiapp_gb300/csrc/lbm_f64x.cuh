@@ -243,6 +243,113 @@ __host__ __device__ __forceinline__ df df_sqr_u(df a)
    return {p, e};
 }
 
+// ------------------------------------------- two float pairs at a time
+// sm_103a's packed FP32 instructions do two independent IEEE operations on a
+// 64-bit register pair: the same FP32 rate (2 cycles per warp instruction and
+// sub-partition instead of 1) from half the issue slots, with negations folded
+// into the operands.  The step kernels are bound by issue slots, so the
+// double-float work runs on two directions at a time.  Each half rounds as the
+// scalar instruction does: the results are the scalar form's, bit for bit.
+struct f2 {
+   float x, y;
+};
+
+__host__ __device__ __forceinline__ f2 dup2(float a) { return {a, a}; }
+__host__ __device__ __forceinline__ f2 neg2(f2 a) { return {-a.x, -a.y}; }
+
+#define LBM_PACKED_BINARY(NAME, OP, SCALAR)                                                                     \
+   __host__ __device__ __forceinline__ f2 NAME(f2 a, f2 b)                                                      \
+   {                                                                                                            \
+      LBM_PACKED_BODY(OP, SCALAR)                                                                               \
+   }
+#ifdef __CUDA_ARCH__
+#define LBM_PACKED_BODY(OP, SCALAR)                                                                             \
+   f2 r;                                                                                                        \
+   asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t" OP " d, a, b;\n\t"        \
+       "mov.b64 {%0, %1}, d;\n\t}"                                                                              \
+       : "=f"(r.x), "=f"(r.y)                                                                                   \
+       : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));                                                               \
+   return r;
+#else
+#define LBM_PACKED_BODY(OP, SCALAR) return {SCALAR(a.x, b.x), SCALAR(a.y, b.y)};
+#endif
+LBM_PACKED_BINARY(add2, "add.rn.f32x2", fadd)
+LBM_PACKED_BINARY(sub2, "sub.rn.f32x2", fsub)
+LBM_PACKED_BINARY(mul2, "mul.rn.f32x2", fmul)
+LBM_PACKED_BINARY(add2_rz, "add.rz.f32x2", fadd_rz)
+#undef LBM_PACKED_BINARY
+#undef LBM_PACKED_BODY
+
+__host__ __device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c)
+{
+#ifdef __CUDA_ARCH__
+   f2 r;
+   asm("{\n\t.reg .b64 a, b, c, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
+       "fma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
+       : "=f"(r.x), "=f"(r.y)
+       : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+   return r;
+#else
+   return {ffma(a.x, b.x, c.x), ffma(a.y, b.y, c.y)};
+#endif
+}
+
+struct df2 {
+   f2 h, l;
+};
+
+__host__ __device__ __forceinline__ df2 dup(df a) { return {dup2(a.h), dup2(a.l)}; }
+__host__ __device__ __forceinline__ df2 pack(df a, df b) { return {{a.h, b.h}, {a.l, b.l}}; }
+__host__ __device__ __forceinline__ df2 df2_neg(df2 a) { return {neg2(a.h), neg2(a.l)}; }
+
+__host__ __device__ __forceinline__ df2 two_sum2(f2 a, f2 b)
+{
+   const f2 s = add2(a, b);
+   const f2 bb = sub2(s, a);
+   return {s, add2(sub2(a, sub2(s, bb)), sub2(b, bb))};
+}
+
+__host__ __device__ __forceinline__ df2 fast_two_sum2(f2 a, f2 b)
+{
+   const f2 s = add2(a, b);
+   return {s, sub2(b, sub2(s, a))};
+}
+
+__host__ __device__ __forceinline__ df2 df2_mul_u(df2 a, df2 b)
+{
+   const f2 p = mul2(a.h, b.h);
+   f2 e = fma2(a.h, b.h, neg2(p));
+   e = fma2(a.h, b.l, e);
+   return {p, fma2(a.l, b.h, e)};
+}
+
+__host__ __device__ __forceinline__ df2 df2_sqr_u(df2 a)
+{
+   const f2 p = mul2(a.h, a.h);
+   const f2 e = fma2(a.h, a.h, neg2(p));
+   return {p, fma2(mul2(dup2(2.0f), a.h), a.l, e)};
+}
+
+__host__ __device__ __forceinline__ uint32_t min3u(uint32_t a, uint32_t b, uint32_t c)
+{
+#ifdef __CUDA_ARCH__
+   return __vimin3_u32(a, b, c);
+#else
+   const uint32_t m = a < b ? a : b;
+   return m < c ? m : c;
+#endif
+}
+
+__host__ __device__ __forceinline__ uint32_t max3u(uint32_t a, uint32_t b, uint32_t c)
+{
+#ifdef __CUDA_ARCH__
+   return __vimax3_u32(a, b, c);
+#else
+   const uint32_t m = a > b ? a : b;
+   return m > c ? m : c;
+#endif
+}
+
 // Exact split of a host double constant into a float pair.
 __host__ __device__ __forceinline__ df df_from_double(double d)
 {
@@ -269,6 +376,17 @@ __host__ __device__ __forceinline__ df split(uint64_t bits)
    const uint32_t hb = (funnel_l(lo, hi, 3) + 0x40000000u) & 0x7FFFFFFFu;
    const float scale = bitsf((hb & 0x7F800000u) - (52u << 23));
    return {bitsf(hb), fmul(u2f_rn(lo & 0x1FFFFFFFu), scale)};
+}
+
+// split() of two doubles of the fast path's range [2^-32, 1), whose exponents
+// (991..1022) have the two bits that the re-biasing takes off both set.
+__host__ __device__ __forceinline__ df2 split2(uint64_t b0, uint64_t b1)
+{
+   const uint32_t lo0 = (uint32_t)b0, lo1 = (uint32_t)b1;
+   const uint32_t h0 = funnel_l(lo0, (uint32_t)(b0 >> 32), 3) & 0x3FFFFFFFu;
+   const uint32_t h1 = funnel_l(lo1, (uint32_t)(b1 >> 32), 3) & 0x3FFFFFFFu;
+   const f2 scale = {bitsf((h0 & 0x7F800000u) - (52u << 23)), bitsf((h1 & 0x7F800000u) - (52u << 23))};
+   return {{bitsf(h0), bitsf(h1)}, mul2({u2f_rn(lo0 & 0x1FFFFFFFu), u2f_rn(lo1 & 0x1FFFFFFFu)}, scale)};
 }
 
 // Fixed-point image of a positive double f in [2^-32, 1) for the moment
@@ -308,18 +426,18 @@ __host__ __device__ __forceinline__ uint32_t f2u_rn(float x)
 #endif
 }
 
-// Running check of the result patterns of one cell: the largest
-// sb - pattern(2^-75) as unsigned (a result below 2^-75 wraps around, a
-// negative or NaN one lands above the bound).
+// Running check of the result patterns of one cell: the smallest and the
+// largest as unsigned integers (a negative or NaN result lands above the
+// bound), two results at a time with three-input minima and maxima.
 struct JoinRange {
-   uint32_t worst = 0u;
-   __host__ __device__ __forceinline__ void add(uint32_t sb)
+   uint32_t least = 0x3F000000u, most = 0x3F000000u;
+   __host__ __device__ __forceinline__ void add(uint32_t s0, uint32_t s1)
    {
-      const uint32_t d = sb - 0x1A000000u;
-      worst = worst > d ? worst : d;
+      least = min3u(least, s0, s1);
+      most = max3u(most, s0, s1);
    }
    // 2^-75 <= S < 1 for every result
-   __host__ __device__ __forceinline__ bool ok() const { return worst < 0x3F800000u - 0x1A000000u; }
+   __host__ __device__ __forceinline__ bool ok() const { return least >= 0x1A000000u && most < 0x3F800000u; }
 };
 
 // Double pattern of h + l (positive):
@@ -335,15 +453,33 @@ struct JoinRange {
 //        the float part and the exponent when N reaches 2^29): within about
 //        33 double ulps of h + l.
 // S's pattern goes into `range`; the result is valid when range.ok().
+__host__ __device__ __forceinline__ uint64_t join_bits(uint32_t sb, float n)
+{
+   return (((uint64_t)sb << 29) + ((uint64_t)0x38000000u << 32)) + f2u_rn(n);
+}
+
 __host__ __device__ __forceinline__ uint64_t join(df v, JoinRange& range)
 {
    const float S = fadd_rz(v.h, v.l);
    const float E = fsub(v.l, fsub(S, v.h));
    const uint32_t sb = fbits(S);
-   range.add(sb);
+   range.add(sb, sb);
    const float scale = bitsf(0x99000000u - (sb & 0x7F800000u));  // 2^(52 - e(S))
-   const uint32_t n = f2u_rn(fmul(E, scale));
-   return (((uint64_t)sb << 29) + ((uint64_t)0x38000000u << 32)) + n;
+   return join_bits(sb, fmul(E, scale));
+}
+
+// join() of two results.
+struct Pattern2 {
+   uint64_t a, b;
+};
+__host__ __device__ __forceinline__ Pattern2 join2(df2 v, JoinRange& range)
+{
+   const f2 S = add2_rz(v.h, v.l);
+   const f2 E = sub2(v.l, sub2(S, v.h));
+   const uint32_t s0 = fbits(S.x), s1 = fbits(S.y);
+   range.add(s0, s1);
+   const f2 n = mul2(E, {bitsf(0x99000000u - (s0 & 0x7F800000u)), bitsf(0x99000000u - (s1 & 0x7F800000u))});
+   return {join_bits(s0, n.x), join_bits(s1, n.y)};
 }
 
 __host__ __device__ __forceinline__ double as_double(uint64_t b)
@@ -454,19 +590,79 @@ __host__ __device__ constexpr int pair_dir(int Q, int p)
 // Fast-path validity thresholds (high words of the doubles).
 constexpr uint32_t kHiQuarter = (uint32_t)(1023 - 2) << 20;   // 0.25
 
-template <int Q, class Again>
-__host__ __device__ __forceinline__ x64::df input_pair(const x64::df (&f)[Q], const Again& again, int s)
-{
-   if constexpr (Again::kRefetch) return again(s);
-   else return f[s];
-}
-
-// Input policy of the fast path that splits the inputs once and keeps the
-// pairs in registers.
+// Input policy of the fast path that keeps the input patterns in registers.
 struct KeepInputs {
    static constexpr bool kRefetch = false;
-   __host__ __device__ __forceinline__ x64::df operator()(int) const { return {0.f, 0.f}; }
+   __host__ __device__ __forceinline__ uint64_t raw(int) const { return 0; }
 };
+
+// Pattern of input s: kept, or read again.
+template <int Q, class Again>
+__host__ __device__ __forceinline__ uint64_t input_bits(const uint64_t (&bits)[Q], const Again& again, int s)
+{
+   if constexpr (Again::kRefetch) return again.raw(s);
+   else return bits[s];
+}
+
+// Parts of the update that two opposite pairs (s, opp(s)) share, the two pairs
+// in the halves: A +- B is omega eq plus the folded forcing, K and sym the
+// forcing added afterwards (FORCE 1).
+struct PairParts {
+   x64::df2 A, B, K, sym;
+};
+
+// cu = 3 c_s.v; owc = omega w rho, om2wc = (1 - omega/2) w of the pairs' class;
+// K = (1 - omega/2) w 3 c_s.F.  Forcing om2 w (+-cf - fu + cu cf) =
+// +-K + (K cu - om2 w fu).
+template <int FORCE>
+__host__ __device__ __forceinline__ PairParts pair_parts(x64::df2 cu, x64::df2 base, x64::df2 owc, x64::df2 K,
+                                                         x64::df2 om2wc, x64::df2 fu)
+{
+   using namespace x64;
+   PairParts r;
+   const f2 half = dup2(0.5f);
+   // Qp = base + cu^2 / 2
+   const df2 c2h = df2_sqr_u(cu);
+   const df2 qs = fast_two_sum2(base.h, mul2(half, c2h.h));
+   const df2 Qp = {qs.h, add2(qs.l, fma2(half, c2h.l, base.l))};
+   r.A = df2_mul_u(owc, Qp);   // omega * eq, symmetric part
+   r.B = df2_mul_u(owc, cu);   // omega * eq, antisymmetric part
+   r.K = K;
+   if constexpr (FORCE != 0) {
+      const df2 gc = df2_mul_u(K, cu);
+      const df2 wf = df2_mul_u(om2wc, fu);
+      const df2 t3 = two_sum2(gc.h, neg2(wf.h));
+      r.sym = {t3.h, add2(t3.l, sub2(gc.l, wf.l))};
+   }
+   if constexpr (FORCE == 2) {
+      // small force: sym joins the symmetric part (far below it) and K the
+      // antisymmetric part (which may vanish, hence TwoSum)
+      const df2 as = fast_two_sum2(r.A.h, r.sym.h);
+      r.A = {as.h, add2(as.l, add2(r.A.l, r.sym.l))};
+      const df2 bs = two_sum2(r.B.h, K.h);
+      r.B = {bs.h, add2(bs.l, add2(r.B.l, K.l))};
+   }
+   return r;
+}
+
+// Patterns of A + B + (1 - omega) f for two directions (B, K negated for the
+// opposite ones), f their inputs.
+template <int FORCE>
+__host__ __device__ __forceinline__ x64::Pattern2 pair_out(const PairParts& q, x64::df2 B, x64::df2 K, x64::df2 f,
+                                                           x64::df2 om1, x64::JoinRange& range)
+{
+   using namespace x64;
+   const df2 tp = fast_two_sum2(q.A.h, B.h);
+   const df2 a = df2_mul_u(om1, f);
+   const df2 t = two_sum2(tp.h, a.h);
+   df2 out = {t.h, add2(t.l, add2(tp.l, add2(add2(q.A.l, B.l), a.l)))};
+   if constexpr (FORCE == 1) {
+      const df2 fr = two_sum2(K.h, q.sym.h);
+      const df2 t2 = two_sum2(out.h, fr.h);
+      out = {t2.h, add2(t2.l, add2(out.l, add2(fr.l, add2(K.l, q.sym.l))))};
+   }
+   return join2(out, range);
+}
 
 // The fast-path collision on one cell.  bits[] holds the Q input patterns in
 // direction order; each output pattern is handed to emit(s, pattern).
@@ -479,19 +675,18 @@ struct KeepInputs {
 //     (1 - uu/2 + cu^2/2) +- cu keep their larger operand first;
 //   * outputs inside [2^-75, 1).
 // Work is organised by opposite pairs (s, opp(s)): cu, the quadratic term and
-// the omega*w*rho products are shared, since cu(opp) = -cu(s).
+// the omega*w*rho products are shared, since cu(opp) = -cu(s).  Two pairs of one
+// weight class go through the packed instructions together; the third axis pair
+// (z) runs alone, its two directions in the halves.
 // FORCE is the forcing form of force_mode() (0 none, 1 added after the
-// equilibrium, 2 folded into it); Again supplies the inputs' float pairs for
-// the (1 - omega) f term (KeepInputs, or a second read from shared memory).
+// equilibrium, 2 folded into it); Again supplies the inputs of the
+// (1 - omega) f term (KeepInputs, or a second read from shared memory).
 //
-// ROLLED (D3Q27): the 13 opposite pairs run in three loops over the pair
-// classes (axes, planar and body diagonals) instead of unrolled, with the same
-// operations in the same order, so the same bits.  The unrolled D3Q27 path
-// runs about 2,700 instructions per cell, more code than the instruction cache
-// holds; rolled, the pair code exists once per class instead of once per
-// pair.  The direction and its velocity are then run-time
-// values: outputs go to emit.put(s, opp(s), c_s, pattern), and Kf points at
-// the per-direction forcing constants (float pairs, direction-indexed).
+// ROLLED (D3Q27): the planar and body diagonals run in loops over their packed
+// pairs instead of unrolled, with the same operations in the same order, so the
+// same bits.  The direction and its velocity are then run-time values: outputs
+// go to emit.put(s, opp(s), c_s, pattern), and Kf points at the per-direction
+// forcing constants (float pairs, direction-indexed).
 template <int Q, int FORCE, class Emit, class Again, bool ROLLED = false>
 __host__ __device__ __forceinline__ bool collide_f64x_fast_emit(const uint64_t (&bits)[Q], const x64::Consts& k,
                                                                int compat, Emit& emit, const Again& again,
@@ -502,37 +697,31 @@ __host__ __device__ __forceinline__ bool collide_f64x_fast_emit(const uint64_t (
    constexpr int NP = (Q - 1) / 2;
    uint32_t hmin = 0xFFFFFFFFu, hmax = 0;
 #pragma unroll
-   for (int s = 0; s < Q; s++) {
-      if (s == R) continue;
-      const uint32_t hi = (uint32_t)(bits[s] >> 32);
-      hmin = hmin < hi ? hmin : hi;
-      hmax = hmax > hi ? hmax : hi;
+   for (int q = 0; q < NP; q++) {
+      const int s = pair_dir(Q, q);
+      const uint32_t hs = (uint32_t)(bits[s] >> 32), ho = (uint32_t)(bits[lat_opp(Q, s)] >> 32);
+      hmin = min3u(hmin, hs, ho);
+      hmax = max3u(hmax, hs, ho);
    }
    const uint32_t hr = (uint32_t)(bits[R] >> 32);
    if (hmin < kHiMin || hmax >= kHiQuarter || hr < kHiQuarter || hr >= kHiMax) return false;
 
-   // Float pairs of the inputs for the update's (1 - omega) f term: split
-   // here and kept, or made again from a second read of the inputs.
-   df f[Q];
-   if constexpr (!Again::kRefetch) {
-#pragma unroll
-      for (int s = 0; s < Q; s++) f[s] = split(bits[s]);
-   }
-
    // rho and j = sum c_s f_s from the exact sums of the fixed-point images
-   // floor(f * 2^53); rho < 2 is checked (rho's top word below 2^22).
-   // One pass: each image goes straight into the four sums.
-   uint64_t rho_x = (uint64_t)(Q / 2);   // mean truncation loss, half a unit per population
+   // floor(f * 2^53); rho < 2 is checked (rho's top word below 2^22).  One
+   // pass: each pair's images go straight into the sums, j by their difference.
+   uint64_t rho_x = fixed53(bits[R]) + (uint64_t)(Q / 2);   // mean truncation loss, half a unit per population
    int64_t jx[3] = {0, 0, 0};
 #pragma unroll
-   for (int s = 0; s < Q; s++) {
-      const uint64_t X = fixed53(bits[s]);
-      rho_x += X;
+   for (int q = 0; q < NP; q++) {
+      const int s = pair_dir(Q, q);
+      const uint64_t X = fixed53(bits[s]), Y = fixed53(bits[lat_opp(Q, s)]);
+      const int64_t D = (int64_t)(X - Y);
+      rho_x += X + Y;
 #pragma unroll
       for (int d = 0; d < 3; d++) {
          const int c = lat_c(Q, s, d);
-         if (c > 0) jx[d] += (int64_t)X;
-         if (c < 0) jx[d] -= (int64_t)X;
+         if (c > 0) jx[d] += D;
+         if (c < 0) jx[d] -= D;
       }
    }
    if ((rho_x >> 32) >= (1u << 22)) return false;
@@ -581,17 +770,13 @@ __host__ __device__ __forceinline__ bool collide_f64x_fast_emit(const uint64_t (
       fu = df_add(fu, df_mul_u(k.F3[2], v[2]));
    }
 
-   df owr[4];
-#pragma unroll
-   for (int cls = 0; cls < 4; cls++) owr[cls] = df_mul_u(k.ow[cls], rho);
-
    // Each output goes to emit(s, pattern) as soon as it is made; the return
    // value says whether all of them passed the range check (if not, the
    // caller overwrites every one with the exact result).
    JoinRange range;
    // rest direction: P = base
    {
-      df A = df_mul_u(owr[0], base);
+      df A = df_mul_u(df_mul_u(k.ow[0], rho), base);
       if (FORCE == 2) {
          // -(1 - omega/2) wf fu (wf = 1/36 with the Unroll-kernel weights),
          // folded into the equilibrium term
@@ -599,7 +784,7 @@ __host__ __device__ __forceinline__ bool collide_f64x_fast_emit(const uint64_t (
          const df t2 = fast_two_sum(A.h, -fr.h);
          A = {t2.h, fadd(t2.l, fsub(A.l, fr.l))};
       }
-      const df a = df_mul_u(k.om1, input_pair(f, again, R));
+      const df a = df_mul_u(k.om1, split(input_bits(bits, again, R)));
       const df t = two_sum(A.h, a.h);
       df out = {t.h, fadd(t.l, fadd(A.l, a.l))};
       if (FORCE == 1) {
@@ -610,156 +795,111 @@ __host__ __device__ __forceinline__ bool collide_f64x_fast_emit(const uint64_t (
       }
       emit(R, join(out, range));
    }
+
+   const df2 base2 = dup(base), fu2 = dup(fu), om1 = dup(k.om1);
+   auto inputs = [&](int a, int b) { return split2(input_bits(bits, again, a), input_bits(bits, again, b)); };
+   auto forcing = [&](int s) {
+      if constexpr (FORCE == 0) return df{0.f, 0.f};
+      else if constexpr (ROLLED) return df{Kf[s][0], Kf[s][1]};
+      else return k.Kf[s];
+   };
+   // Patterns of the pairs (s1, o1), (s2, o2) of one class with cu = (3 c_s1.v,
+   // 3 c_s2.v): out(sign) gives those of s1, s2 (+) or o1, o2 (-).
+   struct Outs {
+      Pattern2 s, o;
+   };
+   auto pairs = [&](const df2 cu, const df2 owc, const df om2wc, int s1, int o1, int s2, int o2) {
+      const PairParts q = pair_parts<FORCE>(cu, base2, owc, pack(forcing(s1), forcing(s2)), dup(om2wc), fu2);
+      Outs r;
+      r.s = pair_out<FORCE>(q, q.B, q.K, inputs(s1, s2), om1, range);
+      r.o = pair_out<FORCE>(q, df2_neg(q.B), df2_neg(q.K), inputs(o1, o2), om1, range);
+      return r;
+   };
+   // axes: (0,1) and (2,3) together, (4,5) with its two directions in the halves
+   {
+      const df2 ow1 = dup(df_mul_u(k.ow[1], rho));
+      const Outs r = pairs(pack(v3[0], v3[1]), ow1, k.om2w[1], 0, 1, 2, 3);
+      const df K = forcing(4);
+      const PairParts q = pair_parts<FORCE>(pack(v3[2], df_neg(v3[2])), base2, ow1, pack(K, df_neg(K)),
+                                            dup(k.om2w[1]), fu2);
+      const Pattern2 z = pair_out<FORCE>(q, q.B, q.K, inputs(4, 5), om1, range);
+      if constexpr (ROLLED) {
+         emit.put(0, 1, 1, 0, 0, r.s.a);
+         emit.put(2, 3, 0, 1, 0, r.s.b);
+         emit.put(1, 0, -1, 0, 0, r.o.a);
+         emit.put(3, 2, 0, -1, 0, r.o.b);
+         emit.put(4, 5, 0, 0, 1, z.a);
+         emit.put(5, 4, 0, 0, -1, z.b);
+      } else {
+         emit(0, r.s.a);
+         emit(2, r.s.b);
+         emit(1, r.o.a);
+         emit(3, r.o.b);
+         emit(4, z.a);
+         emit(5, z.b);
+      }
+   }
+   // cu = a + b in float pairs (TwoSum-based, left unnormalised)
+   auto sum = [](const df2 a, const df2 b) {
+      const df2 t = two_sum2(a.h, b.h);
+      return df2{t.h, add2(t.l, add2(a.l, b.l))};
+   };
+   // planar diagonals (6,11) (7,10), (8,13) (9,12), (14,17) (15,16):
+   // c = e_a + e_b and e_a - e_b, a < b
+   const df2 ow2 = dup(df_mul_u(k.ow[2], rho));
    if constexpr (ROLLED) {
-      static_assert(Q == 27, "the pair-class loops follow the D3Q27 direction order");
-      // One pair (s, o = opp(s)) with c_s = (cx, cy, cz), cu = 3 c_s.v and the
-      // class constants: the unrolled loop's body below, operation for operation.
-      auto pair = [&](int s, int o, int cx, int cy, int cz, const df cu, const df owc, const df om2wc) {
-         const df c2h = df_sqr_u(cu);
-         const df qs = fast_two_sum(base.h, 0.5f * c2h.h);
-         const df Qp = {qs.h, fadd(qs.l, fadd(base.l, 0.5f * c2h.l))};
-         df A = df_mul_u(owc, Qp);
-         df B = df_mul_u(owc, cu);
-         const df Ks = {Kf[s][0], Kf[s][1]};
-         df sym = {0.f, 0.f};
-         if (FORCE) {
-            const df gc = df_mul_u(Ks, cu);
-            const df wf = df_mul_u(om2wc, fu);
-            const df t3 = two_sum(gc.h, -wf.h);
-            sym = {t3.h, fadd(t3.l, fsub(gc.l, wf.l))};
-         }
-         if (FORCE == 2) {
-            const df as = fast_two_sum(A.h, sym.h);
-            A = {as.h, fadd(as.l, fadd(A.l, sym.l))};
-            const df bs = two_sum(B.h, Ks.h);
-            B = {bs.h, fadd(bs.l, fadd(B.l, Ks.l))};
-         }
-         {
-            const df tp = fast_two_sum(A.h, B.h);
-            const df a = df_mul_u(k.om1, input_pair(f, again, s));
-            const df t = two_sum(tp.h, a.h);
-            df out = {t.h, fadd(t.l, fadd(tp.l, fadd(fadd(A.l, B.l), a.l)))};
-            if (FORCE == 1) {
-               const df fr = two_sum(Ks.h, sym.h);
-               const df t2 = two_sum(out.h, fr.h);
-               out = {t2.h, fadd(t2.l, fadd(out.l, fadd(fr.l, fadd(Ks.l, sym.l))))};
-            }
-            emit.put(s, o, cx, cy, cz, join(out, range));
-         }
-         {
-            const df tm = fast_two_sum(A.h, -B.h);
-            const df a = df_mul_u(k.om1, input_pair(f, again, o));
-            const df t = two_sum(tm.h, a.h);
-            df out = {t.h, fadd(t.l, fadd(tm.l, fadd(fsub(A.l, B.l), a.l)))};
-            if (FORCE == 1) {
-               const df fr = two_sum(sym.h, -Ks.h);
-               const df t2 = two_sum(out.h, fr.h);
-               out = {t2.h, fadd(t2.l, fadd(out.l, fadd(fr.l, fsub(sym.l, Ks.l))))};
-            }
-            emit.put(o, s, -cx, -cy, -cz, join(out, range));
-         }
-      };
-      // axes: (0,1) (2,3) (4,5), c = e_d, cu = 3 v_d
+      static_assert(Q == 27, "the loops follow the D3Q27 direction order");
 #pragma unroll 1
-      for (int d = 0; d < 3; d++) {
-         const df cu = d == 0 ? v3[0] : (d == 1 ? v3[1] : v3[2]);
-         pair(2 * d, 2 * d + 1, d == 0, d == 1, d == 2, cu, owr[1], k.om2w[1]);
-      }
-      // planar diagonals (6,11) (7,10) (8,13) (9,12) (14,17) (15,16):
-      // c = e_a + sign e_b, a < b, sign -1 for the odd j
-#pragma unroll 1
-      for (int j = 0; j < 6; j++) {
-         const int a = j < 4 ? 0 : 1, b = j < 2 ? 1 : 2;
-         const bool neg = (j & 1) != 0;
-         const df va = a == 0 ? v3[0] : v3[1];
-         const df vb = b == 1 ? v3[1] : v3[2];
-         const df t = neg ? df_neg(vb) : vb;
-         const df u2 = two_sum(va.h, t.h);
-         const df cu = {u2.h, fadd(u2.l, fadd(va.l, t.l))};
-         const int sgn = neg ? -1 : 1;
-         const int sd = j < 4 ? 6 + j : 10 + j;
-         const int od = j < 2 ? 11 - j : (j < 4 ? 15 - j : 31 - sd);
-         pair(sd, od, a == 0 ? 1 : 0, a == 1 ? 1 : (b == 1 ? sgn : 0), b == 2 ? sgn : 0, cu, owr[2], k.om2w[2]);
-      }
-      // body diagonals (18,25) (19,24) (20,23) (21,22): c = (1, +-1, +-1)
-#pragma unroll 1
-      for (int j = 0; j < 4; j++) {
-         const bool ny = j >= 2, nz = (j & 1) != 0;
-         const df ty = ny ? df_neg(v3[1]) : v3[1];
-         const df u2 = two_sum(v3[0].h, ty.h);
-         df cu = {u2.h, fadd(u2.l, fadd(v3[0].l, ty.l))};
-         const df tz = nz ? df_neg(v3[2]) : v3[2];
-         const df u3 = two_sum(cu.h, tz.h);
-         cu = {u3.h, fadd(u3.l, fadd(cu.l, tz.l))};
-         pair(18 + j, 25 - j, 1, ny ? -1 : 1, nz ? -1 : 1, cu, owr[3], k.om2w[3]);
+      for (int j = 0; j < 3; j++) {
+         const int a = j < 2 ? 0 : 1, b = j == 0 ? 1 : 2;
+         const df va = a == 0 ? v3[0] : v3[1], vb = b == 1 ? v3[1] : v3[2];
+         const int s1 = j == 0 ? 6 : (j == 1 ? 8 : 14), o1 = j == 0 ? 11 : (j == 1 ? 13 : 17);
+         const int s2 = s1 + 1, o2 = o1 - 1;
+         const int ax = a == 0, ay = a == 1, by = b == 1, bz = b == 2;
+         const Outs r = pairs(sum(dup(va), pack(vb, df_neg(vb))), ow2, k.om2w[2], s1, o1, s2, o2);
+         emit.put(s1, o1, ax, ay + by, bz, r.s.a);
+         emit.put(s2, o2, ax, ay - by, -bz, r.s.b);
+         emit.put(o1, s1, -ax, -ay - by, -bz, r.o.a);
+         emit.put(o2, s2, -ax, by - ay, bz, r.o.b);
       }
    } else {
 #pragma unroll
-      for (int q = 0; q < NP; q++) {
-         const int s = pair_dir(Q, q), o = lat_opp(Q, s);
-         const int c0 = lat_c(Q, s, 0), c1 = lat_c(Q, s, 1), c2 = lat_c(Q, s, 2);
-         const int cls = lat_norm2(Q, s);
-         // cu = 3 c_s.v (two_sum-based, left unnormalised)
-         df cu = {0.f, 0.f};
-         bool first = true;
-         if (c0 != 0) { cu = c0 > 0 ? v3[0] : df_neg(v3[0]); first = false; }
-         if (c1 != 0) {
-            const df t = c1 > 0 ? v3[1] : df_neg(v3[1]);
-            if (first) { cu = t; first = false; }
-            else { const df u2 = two_sum(cu.h, t.h); cu = {u2.h, fadd(u2.l, fadd(cu.l, t.l))}; }
+      for (int j = 0; j < 3; j++) {
+         const int a = j < 2 ? 0 : 1, b = j == 0 ? 1 : 2;
+         const int s1 = j == 0 ? 6 : (j == 1 ? 8 : 14), o1 = lat_opp(Q, s1);
+         const int s2 = s1 + 1, o2 = lat_opp(Q, s2);
+         const Outs r = pairs(sum(dup(v3[a]), pack(v3[b], df_neg(v3[b]))), ow2, k.om2w[2], s1, o1, s2, o2);
+         emit(s1, r.s.a);
+         emit(s2, r.s.b);
+         emit(o1, r.o.a);
+         emit(o2, r.o.b);
+      }
+   }
+   // body diagonals (18,25) (20,23), then (19,24) (21,22): c = (1, +-1, 1), (1, +-1, -1)
+   if constexpr (Q == 27) {
+      const df2 ow3 = dup(df_mul_u(k.ow[3], rho));
+      if constexpr (ROLLED) {
+#pragma unroll 1
+         for (int j = 0; j < 2; j++) {
+            const df2 xy = sum(dup(v3[0]), pack(v3[1], df_neg(v3[1])));
+            const df2 z = dup(j == 0 ? v3[2] : df_neg(v3[2]));
+            const int s1 = 18 + j, o1 = 25 - j, s2 = 20 + j, o2 = 23 - j, cz = j == 0 ? 1 : -1;
+            const Outs r = pairs(sum(xy, z), ow3, k.om2w[3], s1, o1, s2, o2);
+            emit.put(s1, o1, 1, 1, cz, r.s.a);
+            emit.put(s2, o2, 1, -1, cz, r.s.b);
+            emit.put(o1, s1, -1, -1, -cz, r.o.a);
+            emit.put(o2, s2, -1, 1, -cz, r.o.b);
          }
-         if (c2 != 0) {
-            const df t = c2 > 0 ? v3[2] : df_neg(v3[2]);
-            if (first) { cu = t; first = false; }
-            else { const df u2 = two_sum(cu.h, t.h); cu = {u2.h, fadd(u2.l, fadd(cu.l, t.l))}; }
-         }
-         // Qp = base + cu^2 / 2
-         const df c2h = df_sqr_u(cu);
-         const df qs = fast_two_sum(base.h, 0.5f * c2h.h);
-         const df Qp = {qs.h, fadd(qs.l, fadd(base.l, 0.5f * c2h.l))};
-         df A = df_mul_u(owr[cls], Qp);   // omega * eq, symmetric part
-         df B = df_mul_u(owr[cls], cu);   // omega * eq, antisymmetric part
-         // forcing om2 w (+-cf - fu + cu cf) = +-Kf[s] + (Kf[s] cu - om2 w fu), with
-         // Kf[s] = om2 w cf a float pair made on the host
-         df sym = {0.f, 0.f};
-         if (FORCE) {
-            const df gc = df_mul_u(k.Kf[s], cu);
-            const df wf = df_mul_u(k.om2w[cls], fu);
-            const df t3 = two_sum(gc.h, -wf.h);
-            sym = {t3.h, fadd(t3.l, fsub(gc.l, wf.l))};
-         }
-         if (FORCE == 2) {
-            // small force: sym joins the symmetric part (far below it) and
-            // Kf[s] the antisymmetric part (which may vanish, hence TwoSum)
-            const df as = fast_two_sum(A.h, sym.h);
-            A = {as.h, fadd(as.l, fadd(A.l, sym.l))};
-            const df bs = two_sum(B.h, k.Kf[s].h);
-            B = {bs.h, fadd(bs.l, fadd(B.l, k.Kf[s].l))};
-         }
-         // s: A + B ; opp(s): A - B ; then + (1 - omega) f
-         {
-            const df tp = fast_two_sum(A.h, B.h);
-            const df a = df_mul_u(k.om1, input_pair(f, again, s));
-            const df t = two_sum(tp.h, a.h);
-            df out = {t.h, fadd(t.l, fadd(tp.l, fadd(fadd(A.l, B.l), a.l)))};
-            if (FORCE == 1) {
-               const df fr = two_sum(k.Kf[s].h, sym.h);
-               const df t2 = two_sum(out.h, fr.h);
-               out = {t2.h, fadd(t2.l, fadd(out.l, fadd(fr.l, fadd(k.Kf[s].l, sym.l))))};
-            }
-            emit(s, join(out, range));
-         }
-         {
-            const df tm = fast_two_sum(A.h, -B.h);
-            const df a = df_mul_u(k.om1, input_pair(f, again, o));
-            const df t = two_sum(tm.h, a.h);
-            df out = {t.h, fadd(t.l, fadd(tm.l, fadd(fsub(A.l, B.l), a.l)))};
-            if (FORCE == 1) {
-               const df fr = two_sum(sym.h, -k.Kf[s].h);
-               const df t2 = two_sum(out.h, fr.h);
-               out = {t2.h, fadd(t2.l, fadd(out.l, fadd(fr.l, fsub(sym.l, k.Kf[s].l))))};
-            }
-            emit(o, join(out, range));
+      } else {
+         const df2 xy = sum(dup(v3[0]), pack(v3[1], df_neg(v3[1])));
+#pragma unroll
+         for (int j = 0; j < 2; j++) {
+            const int s1 = 18 + j, o1 = 25 - j, s2 = 20 + j, o2 = 23 - j;
+            const Outs r = pairs(sum(xy, dup(j == 0 ? v3[2] : df_neg(v3[2]))), ow3, k.om2w[3], s1, o1, s2, o2);
+            emit(s1, r.s.a);
+            emit(s2, r.s.b);
+            emit(o1, r.o.a);
+            emit(o2, r.o.b);
          }
       }
    }
@@ -848,7 +988,6 @@ struct AgainFromShared {
       asm volatile("ld.shared.u64 %0, [%1];\n" : "=l"(v) : "r"(addr + 256u * (uint32_t)s));
       return v;
    }
-   __device__ __forceinline__ x64::df operator()(int s) const { return x64::split(raw(s)); }
 };
 
 // collide_f64x for inputs that stay in shared memory (direction s at in[32 s]),
