@@ -128,25 +128,25 @@ __host__ __device__ __forceinline__ float frcp(float a)
 #endif
 }
 
-// High 32 bits of ((hi:lo) << n), 0 <= n < 32.
+// High 32 bits of ((hi:lo) << n), n modulo 32.
 __host__ __device__ __forceinline__ uint32_t funnel_l(uint32_t lo, uint32_t hi, uint32_t n)
 {
 #ifdef __CUDA_ARCH__
    return __funnelshift_l(lo, hi, n);
 #else
    const uint64_t v = ((uint64_t)hi << 32) | lo;
-   return (uint32_t)((v << n) >> 32);
+   return (uint32_t)((v << (n & 31u)) >> 32);
 #endif
 }
 
-// Low 32 bits of ((hi:lo) >> n), 0 <= n < 32.
+// Low 32 bits of ((hi:lo) >> n), n modulo 32.
 __host__ __device__ __forceinline__ uint32_t funnel_r(uint32_t lo, uint32_t hi, uint32_t n)
 {
 #ifdef __CUDA_ARCH__
    return __funnelshift_r(lo, hi, n);
 #else
    const uint64_t v = ((uint64_t)hi << 32) | lo;
-   return (uint32_t)(v >> n);
+   return (uint32_t)(v >> (n & 31u));
 #endif
 }
 
@@ -393,13 +393,14 @@ __host__ __device__ __forceinline__ df2 split2(uint64_t b0, uint64_t b1)
 // sums: floor(f * 2^53) as a 64-bit integer, the 53-bit mantissa (with its
 // implicit bit) shifted right by k = 1022 - E, in [0, 31] for that range.
 // Sums of these images are exact; the truncation loses less than 2^-53 per
-// population (its mean, half a unit, is added back to rho).
+// population (its mean, half a unit, is added back to rho).  For an f outside
+// that range the result means nothing.
 __host__ __device__ __forceinline__ uint64_t fixed53(uint64_t bits)
 {
    const uint32_t lo = (uint32_t)bits, hi = (uint32_t)(bits >> 32);
    const uint32_t mh = (hi & 0x000FFFFFu) | 0x00100000u;
    const uint32_t k = 1022u - (hi >> 20);
-   return ((uint64_t)(mh >> k) << 32) | funnel_r(lo, mh, k);
+   return ((uint64_t)funnel_r(mh, 0u, k) << 32) | funnel_r(lo, mh, k);
 }
 
 // Float pair of v * 2^-53 for a signed 64-bit v with |v| < 2^54.  The top
@@ -549,6 +550,14 @@ inline void set_collision_constants(KParams& p, int Q, double omega, const doubl
       p.Ff[d] = (float)force[d];
    }
    p.compat = compat;
+   for (int d = 0; d < 3; d++) p.half_F[d] = 0.5 * force[d];
+   for (int q = 0, s = 0; s < Q; s++) {
+      if (s >= lat_opp(Q, s)) continue;
+      // c_s.F as the reference sums it (its zero terms add +-0), then times 3
+      double acc = 0.0;
+      for (int d = 0; d < 3; d++) acc += lat_c(Q, s, d) * force[d];
+      p.cf3[q++] = 3.0 * acc;
+   }
    auto split = [](double d, float* out) {
       const float hi = (float)d;
       out[0] = hi;
@@ -695,36 +704,34 @@ __host__ __device__ __forceinline__ bool collide_f64x_fast_emit(const uint64_t (
    using namespace x64;
    constexpr int R = lat_rest(Q);
    constexpr int NP = (Q - 1) / 2;
+   // One pass over the inputs: the range of their high words, and rho and
+   // j = sum c_s f_s from the exact sums of the fixed-point images
+   // floor(f * 2^53), j by each pair's difference.  An input outside the range
+   // makes meaningless sums, which are not used: so no input has to stay in a
+   // register until the checks are done.
    uint32_t hmin = 0xFFFFFFFFu, hmax = 0;
-#pragma unroll
-   for (int q = 0; q < NP; q++) {
-      const int s = pair_dir(Q, q);
-      const uint32_t hs = (uint32_t)(bits[s] >> 32), ho = (uint32_t)(bits[lat_opp(Q, s)] >> 32);
-      hmin = min3u(hmin, hs, ho);
-      hmax = max3u(hmax, hs, ho);
-   }
-   const uint32_t hr = (uint32_t)(bits[R] >> 32);
-   if (hmin < kHiMin || hmax >= kHiQuarter || hr < kHiQuarter || hr >= kHiMax) return false;
-
-   // rho and j = sum c_s f_s from the exact sums of the fixed-point images
-   // floor(f * 2^53); rho < 2 is checked (rho's top word below 2^22).  One
-   // pass: each pair's images go straight into the sums, j by their difference.
    uint64_t rho_x = fixed53(bits[R]) + (uint64_t)(Q / 2);   // mean truncation loss, half a unit per population
    int64_t jx[3] = {0, 0, 0};
 #pragma unroll
    for (int q = 0; q < NP; q++) {
       const int s = pair_dir(Q, q);
-      const uint64_t X = fixed53(bits[s]), Y = fixed53(bits[lat_opp(Q, s)]);
-      const int64_t D = (int64_t)(X - Y);
+      const uint64_t bs = bits[s], bo = bits[lat_opp(Q, s)];
+      hmin = min3u(hmin, (uint32_t)(bs >> 32), (uint32_t)(bo >> 32));
+      hmax = max3u(hmax, (uint32_t)(bs >> 32), (uint32_t)(bo >> 32));
+      const uint64_t X = fixed53(bs), Y = fixed53(bo);
+      const uint64_t D = X - Y;
       rho_x += X + Y;
 #pragma unroll
       for (int d = 0; d < 3; d++) {
          const int c = lat_c(Q, s, d);
-         if (c > 0) jx[d] += D;
-         if (c < 0) jx[d] -= D;
+         if (c > 0) jx[d] = (int64_t)((uint64_t)jx[d] + D);
+         if (c < 0) jx[d] = (int64_t)((uint64_t)jx[d] - D);
       }
    }
-   if ((rho_x >> 32) >= (1u << 22)) return false;
+   const uint32_t hr = (uint32_t)(bits[R] >> 32);
+   // rho < 2: its top word is below 2^22
+   if (hmin < kHiMin || hmax >= kHiQuarter || hr < kHiQuarter || hr >= kHiMax || (rho_x >> 32) >= (1u << 22))
+      return false;
    df j[3];
 #pragma unroll
    for (int d = 0; d < 3; d++) {
@@ -951,17 +958,6 @@ __device__ __forceinline__ x64::Consts collide_consts(const KParams& p)
    return k;
 }
 
-template <int Q>
-__device__ __forceinline__ void collide_exact_bits(uint64_t (&bits)[Q], const KParams& p)
-{
-   double d[Q], o[Q];
-#pragma unroll
-   for (int s = 0; s < Q; s++) d[s] = x64::as_double(bits[s]);
-   collide_f64<Q>(d, o, p.F[0], p.F[1], p.F[2], 0.0, p);
-#pragma unroll
-   for (int s = 0; s < Q; s++) bits[s] = x64::double_bits(o[s]);
-}
-
 // F64X cell update with a uniform force: fast path, else the exact IEEE
 // double collision.
 template <int Q>
@@ -972,7 +968,12 @@ __device__ __forceinline__ void collide_f64x(uint64_t (&bits)[Q], const KParams&
                      : p.forced    ? collide_f64x_fast<Q, 1>(bits, k, p.compat)
                                    : collide_f64x_fast<Q, 0>(bits, k, p.compat);
    if (fast) return;
-   collide_exact_bits<Q>(bits, p);
+   double o[Q];
+   auto in = [&](int s) { return x64::as_double(bits[s]); };
+   auto keep = [&](int s, double v) { o[s] = v; };
+   collide_f64_uniform<Q>(in, keep, 0.0, p);
+#pragma unroll
+   for (int s = 0; s < Q; s++) bits[s] = x64::double_bits(o[s]);
 }
 
 // Input pattern s read again from shared memory (direction s at byte 256 s
@@ -1014,11 +1015,9 @@ __device__ __forceinline__ void collide_f64x_shared_emit(const unsigned long lon
       : p.forced    ? collide_f64x_fast_emit<Q, 1, Emit, A, ROLLED>(bits, k, p.compat, emit, again, p.x_Kf)
                     : collide_f64x_fast_emit<Q, 0, Emit, A, ROLLED>(bits, k, p.compat, emit, again, p.x_Kf);
    if (fast) return;
-#pragma unroll
-   for (int s = 0; s < Q; s++) bits[s] = again.raw(s);
-   collide_exact_bits<Q>(bits, p);
-#pragma unroll
-   for (int s = 0; s < Q; s++) emit(s, bits[s]);
+   auto input = [&](int s) { return x64::as_double(again.raw(s)); };
+   auto out = [&](int s, double v) { emit(s, x64::double_bits(v)); };
+   collide_f64_uniform<Q>(input, out, 0.0, p);
 }
 
 }  // namespace lbm

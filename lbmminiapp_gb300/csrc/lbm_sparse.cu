@@ -94,24 +94,23 @@ __global__ void __launch_bounds__(kSparseThreads, sparse_min_blocks<Q>()) sparse
       else loc[s] = (uint32_t)adj[(size_t)nf * s + ii];
       d[s] = src[loc[s]];
    }
-   double o[Q];
+   auto put = [&](int s, double v) {
+      uint32_t w;
+      if (KIND == K_AA_EVEN || KIND == K_AB_PULL) w = nf * (uint32_t)s + ii;
+      else if (KIND == K_AA_ODD) w = loc[lat_opp(Q, s)];
+      else w = (uint32_t)adj[(size_t)nf * s + ii];
+      dst[w] = v;
+   };
    if constexpr (AR == AR_F64) {
-      collide_f64<Q>(d, o, p.F[0], p.F[1], p.F[2], 0.0, p);
+      auto in = [&](int s) { return d[s]; };
+      collide_f64_uniform<Q>(in, put, 0.0, p);
    } else {
       uint64_t bits[Q];
 #pragma unroll
       for (int s = 0; s < Q; s++) bits[s] = x64::double_bits(d[s]);
       collide_f64x<Q>(bits, p);
 #pragma unroll
-      for (int s = 0; s < Q; s++) o[s] = x64::as_double(bits[s]);
-   }
-#pragma unroll
-   for (int s = 0; s < Q; s++) {
-      uint32_t w;
-      if (KIND == K_AA_EVEN || KIND == K_AB_PULL) w = nf * (uint32_t)s + ii;
-      else if (KIND == K_AA_ODD) w = loc[lat_opp(Q, s)];
-      else w = (uint32_t)adj[(size_t)nf * s + ii];
-      dst[w] = o[s];
+      for (int s = 0; s < Q; s++) put(s, x64::as_double(bits[s]));
    }
 }
 

@@ -165,14 +165,15 @@ __global__ void __launch_bounds__(256) step_kernel(const KParams p, const typena
    const T* sbase = src + ci.c;
    T* dbase = dst + ci.c;
    if constexpr (AR == AR_F64) {
-      double d[Q], o[Q];
+      double d[Q];
 #pragma unroll
       for (int s = 0; s < Q; s++) d[s] = *slot_ptr(sbase, pb, read_access<Q, KIND, LINKS>(ci, lk, s));
       double F0, F1, F2, sp;
       cell_force_f64<FIELDS>(p, ci.c, F0, F1, F2, sp);
-      collide_f64<Q>(d, o, F0, F1, F2, sp, p);
-#pragma unroll
-      for (int s = 0; s < Q; s++) *slot_ptr(dbase, pb, write_access<Q, KIND, LINKS>(ci, lk, s)) = o[s];
+      auto in = [&](int s) { return d[s]; };
+      auto out = [&](int s, double v) { *slot_ptr(dbase, pb, write_access<Q, KIND, LINKS>(ci, lk, s)) = v; };
+      if (FIELDS && p.force_field) collide_f64_emit<Q, XF_CELL>(in, out, F0, F1, F2, sp, p);
+      else collide_f64_uniform<Q>(in, out, sp, p);
    } else if constexpr (AR == AR_F64X) {
       uint64_t bits[Q];
       const unsigned long long* s64 = reinterpret_cast<const unsigned long long*>(sbase);
