@@ -516,12 +516,14 @@ struct Consts {
    df om2w[4];    // (1 - omega/2) w per weight class
    df om2w36;     // (1 - omega/2) / 36 (rest weight of the Q19 AA Unroll kernels)
    float om2;
+   // small-force form (FORCE 3): F / omega, (1 - omega/2) / omega, and per
+   // direction 3/2 F.F - (3 c.F)^2 / 2
+   df Fshift[3];
+   float kappa, E[27];
 };
 
 }  // namespace x64
 
-// Host: the collision constants of a launch (relaxation rate, uniform force,
-// the Q19 AA Unroll rest-weight switch) in double, float and float-pair form.
 // Forcing form of the F64X fast path: 0 no force; 1 any force (the forcing
 // terms are added after the equilibrium with error-free sums); 2 a force small
 // enough, sum |F_d| <= 0.004 omega, for the terms to be folded into the
@@ -537,6 +539,25 @@ inline int force_mode(const double force[3], double omega)
    return fsum <= 0.004 * omega ? 2 : 1;
 }
 
+// Form 3 of the step kernels: the force shifts the velocity.  With
+// k = (1 - omega/2) / (omega rho) and v' = (j + F/omega) / rho = v + k F,
+//   omega eq_s(v) + (1 - omega/2) fdist_s = omega eq_s(v') + omega w rho k^2 E_s,
+//   E_s = 3/2 F.F - (3 c.F)^2 / 2,
+// exactly: the forcing costs one multiply-add per pair instead of about 25
+// double-float operations.  The E term is single precision: with
+// sum |F_d| (1 - omega/2) / omega <= 1e-5 it is below 2^-28 of the equilibrium
+// (rho >= 1/4), its rounding below 2^-51.  Every workload of the benchmark lies
+// there.  Not for the rest weight of the Unroll kernels (compat), which breaks
+// the identity.
+inline bool force_shifts(const double force[3], double omega)
+{
+   double fsum = 0.0;
+   for (int d = 0; d < 3; d++) fsum += force[d] < 0.0 ? -force[d] : force[d];
+   return fsum > 0.0 && fsum * (1.0 - 0.5 * omega) <= 1e-5 * omega;
+}
+
+// Host: the collision constants of a launch (relaxation rate, uniform force,
+// the Q19 AA Unroll rest-weight switch) in double, float and float-pair form.
 inline void set_collision_constants(KParams& p, int Q, double omega, const double force[3], int compat)
 {
    p.omega = omega;
@@ -580,6 +601,14 @@ inline void set_collision_constants(KParams& p, int Q, double omega, const doubl
    for (int d = 0; d < 3; d++) split(3.0 * force[d], p.x_F3[d]);
    split(p.om2 / 36.0, p.x_om2w36);
    p.forced = force_mode(force, omega);
+   if (!compat && force_shifts(force, omega)) p.forced = 3;
+   for (int d = 0; d < 3; d++) split(force[d] / omega, p.x_Fshift[d]);
+   p.x_kappa = (float)((1.0 - 0.5 * omega) / omega);
+   for (int s = 0; s < Q; s++) {
+      const double cf = 3.0 * (lat_c(Q, s, 0) * force[0] + lat_c(Q, s, 1) * force[1] + lat_c(Q, s, 2) * force[2]);
+      const double ff = force[0] * force[0] + force[1] * force[1] + force[2] * force[2];
+      p.x_E[s] = (float)(1.5 * ff - 0.5 * cf * cf);
+   }
 }
 
 // Representative s < opp(s) of the p-th opposite pair (direction order of
@@ -622,10 +651,10 @@ struct PairParts {
 
 // cu = 3 c_s.v; owc = omega w rho, om2wc = (1 - omega/2) w of the pairs' class;
 // K = (1 - omega/2) w 3 c_s.F.  Forcing om2 w (+-cf - fu + cu cf) =
-// +-K + (K cu - om2 w fu).
+// +-K + (K cu - om2 w fu); FORCE 3: kk E = k^2 E_s joins the quadratic term.
 template <int FORCE>
 __host__ __device__ __forceinline__ PairParts pair_parts(x64::df2 cu, x64::df2 base, x64::df2 owc, x64::df2 K,
-                                                         x64::df2 om2wc, x64::df2 fu)
+                                                         x64::df2 om2wc, x64::df2 fu, x64::f2 kk, x64::f2 E)
 {
    using namespace x64;
    PairParts r;
@@ -633,11 +662,13 @@ __host__ __device__ __forceinline__ PairParts pair_parts(x64::df2 cu, x64::df2 b
    // Qp = base + cu^2 / 2
    const df2 c2h = df2_sqr_u(cu);
    const df2 qs = fast_two_sum2(base.h, mul2(half, c2h.h));
-   const df2 Qp = {qs.h, add2(qs.l, fma2(half, c2h.l, base.l))};
+   f2 low = fma2(half, c2h.l, base.l);
+   if constexpr (FORCE == 3) low = fma2(kk, E, low);
+   const df2 Qp = {qs.h, add2(qs.l, low)};
    r.A = df2_mul_u(owc, Qp);   // omega * eq, symmetric part
    r.B = df2_mul_u(owc, cu);   // omega * eq, antisymmetric part
    r.K = K;
-   if constexpr (FORCE != 0) {
+   if constexpr (FORCE == 1 || FORCE == 2) {
       const df2 gc = df2_mul_u(K, cu);
       const df2 wf = df2_mul_u(om2wc, fu);
       const df2 t3 = two_sum2(gc.h, neg2(wf.h));
@@ -687,19 +718,20 @@ __host__ __device__ __forceinline__ x64::Pattern2 pair_out(const PairParts& q, x
 // the omega*w*rho products are shared, since cu(opp) = -cu(s).  Two pairs of one
 // weight class go through the packed instructions together; the third axis pair
 // (z) runs alone, its two directions in the halves.
-// FORCE is the forcing form of force_mode() (0 none, 1 added after the
-// equilibrium, 2 folded into it); Again supplies the inputs of the
+// FORCE is the forcing form (0 none, 1 added after the equilibrium, 2 folded
+// into it, 3 a velocity shift: force_mode(), force_shifts()); Again supplies the inputs of the
 // (1 - omega) f term (KeepInputs, or a second read from shared memory).
 //
 // ROLLED (D3Q27): the planar and body diagonals run in loops over their packed
 // pairs instead of unrolled, with the same operations in the same order, so the
 // same bits.  The direction and its velocity are then run-time values: outputs
-// go to emit.put(s, opp(s), c_s, pattern), and Kf points at the per-direction
-// forcing constants (float pairs, direction-indexed).
+// go to emit.put(s, opp(s), c_s, pattern), and Kf (float pairs) and E point at
+// the per-direction forcing constants.
 template <int Q, int FORCE, class Emit, class Again, bool ROLLED = false>
 __host__ __device__ __forceinline__ bool collide_f64x_fast_emit(const uint64_t (&bits)[Q], const x64::Consts& k,
                                                                int compat, Emit& emit, const Again& again,
-                                                               const float (*Kf)[2] = nullptr)
+                                                               const float (*Kf)[2] = nullptr,
+                                                               const float* E = nullptr)
 {
    using namespace x64;
    constexpr int R = lat_rest(Q);
@@ -751,7 +783,9 @@ __host__ __device__ __forceinline__ bool collide_f64x_fast_emit(const uint64_t (
    df v[3], v3[3];
 #pragma unroll
    for (int d = 0; d < 3; d++) {
-      const df jf = FORCE ? df_add(j[d], {0.5f * k.F[d].h, 0.5f * k.F[d].l}) : j[d];
+      df jf = j[d];
+      if constexpr (FORCE == 3) jf = df_add(j[d], k.Fshift[d]);
+      else if constexpr (FORCE != 0) jf = df_add(j[d], {0.5f * k.F[d].h, 0.5f * k.F[d].l});
       v[d] = df_mul_u(jf, inv);
       const float p = fmul(3.0f, v[d].h);
       v3[d] = fast_two_sum(p, ffma(3.0f, v[d].h, -p) + 3.0f * v[d].l);
@@ -771,7 +805,7 @@ __host__ __device__ __forceinline__ bool collide_f64x_fast_emit(const uint64_t (
    }
    // fu = 3 F.v (float pair; zero without a force)
    df fu = {0.f, 0.f};
-   if (FORCE) {
+   if constexpr (FORCE == 1 || FORCE == 2) {
       fu = df_mul_u(k.F3[0], v[0]);
       fu = df_add(fu, df_mul_u(k.F3[1], v[1]));
       fu = df_add(fu, df_mul_u(k.F3[2], v[2]));
@@ -781,9 +815,14 @@ __host__ __device__ __forceinline__ bool collide_f64x_fast_emit(const uint64_t (
    // value says whether all of them passed the range check (if not, the
    // caller overwrites every one with the exact result).
    JoinRange range;
+   float kk = 0.f;   // k^2 of the velocity shift
+   if constexpr (FORCE == 3) {
+      const float kr = fmul(k.kappa, r0);
+      kk = fmul(kr, kr);
+   }
    // rest direction: P = base
    {
-      df A = df_mul_u(df_mul_u(k.ow[0], rho), base);
+      df A = df_mul_u(df_mul_u(k.ow[0], rho), FORCE == 3 ? df{base.h, ffma(kk, k.E[R], base.l)} : base);
       if (FORCE == 2) {
          // -(1 - omega/2) wf fu (wf = 1/36 with the Unroll-kernel weights),
          // folded into the equilibrium term
@@ -806,9 +845,14 @@ __host__ __device__ __forceinline__ bool collide_f64x_fast_emit(const uint64_t (
    const df2 base2 = dup(base), fu2 = dup(fu), om1 = dup(k.om1);
    auto inputs = [&](int a, int b) { return split2(input_bits(bits, again, a), input_bits(bits, again, b)); };
    auto forcing = [&](int s) {
-      if constexpr (FORCE == 0) return df{0.f, 0.f};
+      if constexpr (FORCE == 0 || FORCE == 3) return df{0.f, 0.f};
       else if constexpr (ROLLED) return df{Kf[s][0], Kf[s][1]};
       else return k.Kf[s];
+   };
+   auto shift = [&](int s) {
+      if constexpr (FORCE != 3) return 0.f;
+      else if constexpr (ROLLED) return E[s];
+      else return k.E[s];
    };
    // Patterns of the pairs (s1, o1), (s2, o2) of one class with cu = (3 c_s1.v,
    // 3 c_s2.v): out(sign) gives those of s1, s2 (+) or o1, o2 (-).
@@ -816,7 +860,8 @@ __host__ __device__ __forceinline__ bool collide_f64x_fast_emit(const uint64_t (
       Pattern2 s, o;
    };
    auto pairs = [&](const df2 cu, const df2 owc, const df om2wc, int s1, int o1, int s2, int o2) {
-      const PairParts q = pair_parts<FORCE>(cu, base2, owc, pack(forcing(s1), forcing(s2)), dup(om2wc), fu2);
+      const PairParts q = pair_parts<FORCE>(cu, base2, owc, pack(forcing(s1), forcing(s2)), dup(om2wc), fu2,
+                                            dup2(kk), {shift(s1), shift(s2)});
       Outs r;
       r.s = pair_out<FORCE>(q, q.B, q.K, inputs(s1, s2), om1, range);
       r.o = pair_out<FORCE>(q, df2_neg(q.B), df2_neg(q.K), inputs(o1, o2), om1, range);
@@ -828,7 +873,7 @@ __host__ __device__ __forceinline__ bool collide_f64x_fast_emit(const uint64_t (
       const Outs r = pairs(pack(v3[0], v3[1]), ow1, k.om2w[1], 0, 1, 2, 3);
       const df K = forcing(4);
       const PairParts q = pair_parts<FORCE>(pack(v3[2], df_neg(v3[2])), base2, ow1, pack(K, df_neg(K)),
-                                            dup(k.om2w[1]), fu2);
+                                            dup(k.om2w[1]), fu2, dup2(kk), dup2(shift(4)));
       const Pattern2 z = pair_out<FORCE>(q, q.B, q.K, inputs(4, 5), om1, range);
       if constexpr (ROLLED) {
          emit.put(0, 1, 1, 0, 0, r.s.a);
@@ -855,7 +900,6 @@ __host__ __device__ __forceinline__ bool collide_f64x_fast_emit(const uint64_t (
    // c = e_a + e_b and e_a - e_b, a < b
    const df2 ow2 = dup(df_mul_u(k.ow[2], rho));
    if constexpr (ROLLED) {
-      static_assert(Q == 27, "the loops follow the D3Q27 direction order");
 #pragma unroll 1
       for (int j = 0; j < 3; j++) {
          const int a = j < 2 ? 0 : 1, b = j == 0 ? 1 : 2;
@@ -938,7 +982,7 @@ __host__ __device__ __forceinline__ bool collide_f64x_fast(uint64_t (&bits)[Q], 
 // F64X cell update with a uniform force: fast path, else the exact IEEE
 // double collision.
 template <int Q>
-__device__ __forceinline__ x64::Consts collide_consts(const KParams& p)
+__host__ __device__ __forceinline__ x64::Consts collide_consts(const KParams& p)
 {
    x64::Consts k;
    k.om1 = {p.x_om1[0], p.x_om1[1]};
@@ -955,6 +999,11 @@ __device__ __forceinline__ x64::Consts collide_consts(const KParams& p)
    for (int c = 0; c < 4; c++) k.om2w[c] = {p.x_om2w[c][0], p.x_om2w[c][1]};
    k.om2w36 = {p.x_om2w36[0], p.x_om2w36[1]};
    k.om2 = p.om2f;
+#pragma unroll
+   for (int d = 0; d < 3; d++) k.Fshift[d] = {p.x_Fshift[d][0], p.x_Fshift[d][1]};
+   k.kappa = p.x_kappa;
+#pragma unroll
+   for (int s = 0; s < Q; s++) k.E[s] = p.x_E[s];
    return k;
 }
 
@@ -964,7 +1013,8 @@ template <int Q>
 __device__ __forceinline__ void collide_f64x(uint64_t (&bits)[Q], const KParams& p)
 {
    const x64::Consts k = collide_consts<Q>(p);
-   const bool fast = p.forced == 2 ? collide_f64x_fast<Q, 2>(bits, k, p.compat)
+   const bool fast = p.forced == 3   ? collide_f64x_fast<Q, 3>(bits, k, p.compat)
+                     : p.forced == 2 ? collide_f64x_fast<Q, 2>(bits, k, p.compat)
                      : p.forced    ? collide_f64x_fast<Q, 1>(bits, k, p.compat)
                                    : collide_f64x_fast<Q, 0>(bits, k, p.compat);
    if (fast) return;
@@ -1011,7 +1061,8 @@ __device__ __forceinline__ void collide_f64x_shared_emit(const unsigned long lon
    const AgainFromShared again{(uint32_t)__cvta_generic_to_shared(in)};
    using A = AgainFromShared;
    const bool fast =
-      p.forced == 2 ? collide_f64x_fast_emit<Q, 2, Emit, A, ROLLED>(bits, k, p.compat, emit, again, p.x_Kf)
+      p.forced == 3   ? collide_f64x_fast_emit<Q, 3, Emit, A, ROLLED>(bits, k, p.compat, emit, again, p.x_Kf, p.x_E)
+      : p.forced == 2 ? collide_f64x_fast_emit<Q, 2, Emit, A, ROLLED>(bits, k, p.compat, emit, again, p.x_Kf)
       : p.forced    ? collide_f64x_fast_emit<Q, 1, Emit, A, ROLLED>(bits, k, p.compat, emit, again, p.x_Kf)
                     : collide_f64x_fast_emit<Q, 0, Emit, A, ROLLED>(bits, k, p.compat, emit, again, p.x_Kf);
    if (fast) return;

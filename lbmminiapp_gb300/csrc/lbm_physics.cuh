@@ -55,7 +55,9 @@ struct KParams {
    float x_F3[3][2];              // 3 F
    float x_om2w[4][2];            // (1 - omega/2) w per weight class
    float x_om2w36[2];             // (1 - omega/2) / 36
-   int forced;                    // uniform force nonzero
+   float x_Fshift[3][2];          // F / omega
+   float x_kappa, x_E[27];        // (1 - omega/2) / omega; 3/2 F.F - (3 c_s.F)^2 / 2 per direction
+   int forced;                    // forcing form of the F64X fast path, 0 without a uniform force
    // Exact FP64 arithmetic: F/2 and 3 c_s.F of the uniform force for the first
    // direction s of each opposite pair, rounded as the reference rounds them.
    double half_F[3];
