@@ -23,10 +23,16 @@ LIB = PKG / "liblbm_gb300.so"
 APP = PKG / "lbm-gb300-app"
 
 SOURCES = [
+    "lbm_step_q27_f64x.cu",
+    "lbm_step_q27_f64.cu",
     "lbm_api.cu",
+    "lbm_step_q27_aa.cu",
+    "lbm_step_q27_ab.cu",
+    "lbm_step_q19_aa.cu",
+    "lbm_step_q19_ab.cu",
+    "lbm_step_q19_f64x.cu",
     "lbm_step_q19_f64.cu",
     "lbm_step_q19_low.cu",
-    "lbm_step_q27_f64.cu",
     "lbm_step_q27_low.cu",
     "lbm_noalloc.cu",
     "lbm_sparse.cu",

@@ -45,23 +45,23 @@ cudaError_t launch_kind(const Launch& L, const KParams& p, const void* src, void
    }
    if constexpr (ST == ST_F64 && AR == AR_F64X) {
       if (L.async && !fields) {
-         const bool ragged = p.nx % 32 != 0;
-         if (links) return ragged ? launch_async<Q, KIND, true, true>(p, L.ag, src, dst, L.stream)
-                                  : launch_async<Q, KIND, true, false>(p, L.ag, src, dst, L.stream);
-         return ragged ? launch_async<Q, KIND, false, true>(p, L.ag, src, dst, L.stream)
-                       : launch_async<Q, KIND, false, false>(p, L.ag, src, dst, L.stream);
+         if constexpr (KIND == K_AA_EVEN || KIND == K_AA_ODD)
+            return launch_async_aa<Q>(KIND, links, p, L.ag, src, dst, L.stream);
+         else
+            return launch_async_ab<Q>(KIND, links, p, L.ag, src, dst, L.stream);
       }
    }
-   // Per-cell fields always use the exact FP64 arithmetic when FP64 is stored.
-   constexpr int ARF = (AR == AR_F64X) ? AR_F64 : AR;
    // Per-cell fields (porosity, force field): 64-bit stride arithmetic only.
    // The plain step kernels get a 32-bit stride variant for planes below 4 GiB.
-   if (fields) {
-      if (links)
-         return launch_overlapped(step_kernel<Q, ST, ARF, KIND, true, true, int64_t>, L.grid, L.block, 0, L.stream, p,
+   // F64X has none (launch_step_q*_f64 takes them to the exact arithmetic).
+   if constexpr (AR != AR_F64X) {
+      if (fields) {
+         if (links)
+            return launch_overlapped(step_kernel<Q, ST, AR, KIND, true, true, int64_t>, L.grid, L.block, 0, L.stream,
+                                     p, s, d);
+         return launch_overlapped(step_kernel<Q, ST, AR, KIND, false, true, int64_t>, L.grid, L.block, 0, L.stream, p,
                                   s, d);
-      return launch_overlapped(step_kernel<Q, ST, ARF, KIND, false, true, int64_t>, L.grid, L.block, 0, L.stream, p, s,
-                               d);
+      }
    }
    if (L.idx32) {
       if (links)
@@ -89,8 +89,10 @@ cudaError_t launch_step_t(int kind, const Launch& L, const KParams& p, const voi
    }
 }
 
-// Defined in lbm_step_q19_f64.cu, lbm_step_q19_low.cu, lbm_step_q27_f64.cu,
-// lbm_step_q27_low.cu.
+// Defined in lbm_step_q19_f64.cu, lbm_step_q19_f64x.cu, lbm_step_q19_low.cu,
+// lbm_step_q27_f64.cu, lbm_step_q27_f64x.cu, lbm_step_q27_low.cu.
+cudaError_t launch_step_q19_f64x(int kind, const Launch& L, const KParams& p, const void* src, void* dst, bool links);
+cudaError_t launch_step_q27_f64x(int kind, const Launch& L, const KParams& p, const void* src, void* dst, bool links);
 cudaError_t launch_step_q19_f64(int arith, int kind, const Launch& L, const KParams& p,
                                 const void* src, void* dst, bool links, bool fields);
 cudaError_t launch_step_q19_low(int storage, int kind, const Launch& L, const KParams& p,

@@ -722,11 +722,14 @@ __host__ __device__ __forceinline__ x64::Pattern2 pair_out(const PairParts& q, x
 // into it, 3 a velocity shift: force_mode(), force_shifts()); Again supplies the inputs of the
 // (1 - omega) f term (KeepInputs, or a second read from shared memory).
 //
-// ROLLED (D3Q27): the planar and body diagonals run in loops over their packed
-// pairs instead of unrolled, with the same operations in the same order, so the
-// same bits.  The direction and its velocity are then run-time values: outputs
-// go to emit.put(s, opp(s), c_s, pattern), and Kf (float pairs) and E point at
-// the per-direction forcing constants.
+// ROLLED: the planar and body diagonals run in loops over their packed pairs
+// instead of unrolled, with the same operations in the same order, so the same
+// bits.  The direction and its velocity are then run-time values: outputs go to
+// emit.put(s, opp(s), c_s, pattern), and Kf (float pairs) and E point at the
+// per-direction forcing constants.  The step kernels run the unrolled form (the
+// loops' smaller code paid only while the scalar form overran the instruction
+// cache: D3Q27 AA even step, 256x128x128: 293 us rolled, 283 us unrolled); the
+// rolled one is its cross-check on the host.
 template <int Q, int FORCE, class Emit, class Again, bool ROLLED = false>
 __host__ __device__ __forceinline__ bool collide_f64x_fast_emit(const uint64_t (&bits)[Q], const x64::Consts& k,
                                                                int compat, Emit& emit, const Again& again,
@@ -1049,9 +1052,12 @@ struct AgainFromShared {
 // over them (the fallback reads its inputs from shared memory): a caller's
 // emit must let a later emit of the same s win, as stores from one thread to
 // one address do.
-// ROLLED: the D3Q27 pair-class loops (collide_f64x_fast_emit), whose outputs
-// go to emit.put.
-template <int Q, bool ROLLED = false, class Emit>
+// FORCE: the launch's forcing form (p.forced), compile-time for no force and for
+// the velocity shift, the forms that nearly every run has: a kernel that holds
+// all four forms' code allocates registers for the worst of them (D3Q19 AA odd
+// step, 256x128x128: 219 us against 211).  kForceOther holds forms 1 and 2.
+constexpr int kForceOther = 1;
+template <int Q, int FORCE, class Emit>
 __device__ __forceinline__ void collide_f64x_shared_emit(const unsigned long long* in, const KParams& p, Emit& emit)
 {
    uint64_t bits[Q];
@@ -1059,16 +1065,15 @@ __device__ __forceinline__ void collide_f64x_shared_emit(const unsigned long lon
    for (int s = 0; s < Q; s++) bits[s] = in[s * 32];
    const x64::Consts k = collide_consts<Q>(p);
    const AgainFromShared again{(uint32_t)__cvta_generic_to_shared(in)};
-   using A = AgainFromShared;
-   const bool fast =
-      p.forced == 3   ? collide_f64x_fast_emit<Q, 3, Emit, A, ROLLED>(bits, k, p.compat, emit, again, p.x_Kf, p.x_E)
-      : p.forced == 2 ? collide_f64x_fast_emit<Q, 2, Emit, A, ROLLED>(bits, k, p.compat, emit, again, p.x_Kf)
-      : p.forced    ? collide_f64x_fast_emit<Q, 1, Emit, A, ROLLED>(bits, k, p.compat, emit, again, p.x_Kf)
-                    : collide_f64x_fast_emit<Q, 0, Emit, A, ROLLED>(bits, k, p.compat, emit, again, p.x_Kf);
+   bool fast;
+   if constexpr (FORCE == kForceOther)
+      fast = p.forced == 2 ? collide_f64x_fast_emit<Q, 2>(bits, k, p.compat, emit, again)
+                           : collide_f64x_fast_emit<Q, 1>(bits, k, p.compat, emit, again);
+   else fast = collide_f64x_fast_emit<Q, FORCE>(bits, k, p.compat, emit, again);
    if (fast) return;
    auto input = [&](int s) { return x64::as_double(again.raw(s)); };
    auto out = [&](int s, double v) { emit(s, x64::double_bits(v)); };
-   collide_f64_uniform<Q>(input, out, 0.0, p);
+   collide_f64_emit<Q, FORCE == 0 ? XF_NONE : XF_UNIFORM>(input, out, 0.0, 0.0, 0.0, 0.0, p);
 }
 
 }  // namespace lbm

@@ -124,8 +124,13 @@ __global__ void __launch_bounds__(kSparseThreads, sparse_min_blocks<Q>()) sparse
 // and each output is stored as the collision makes it.  AA stays race-free
 // under the prefetch: a fluid point's read and write locations are the same
 // set, disjoint from every other point's.
-constexpr int kSparseAsyncWarps = 4;
-constexpr int kSparseAsyncBlocks = 3;
+// Warps per block and blocks per SM: 12 warps at up to 168 registers, D3Q27 in
+// one block so that their shared memory fits the 164 KB carve-out
+// (lbm_step_async.cuh says why that matters).
+template <int Q>
+constexpr int sparse_warps() { return Q == 19 ? 4 : 12; }
+template <int Q>
+constexpr int sparse_blocks() { return Q == 19 ? 3 : 1; }
 
 template <int KIND>
 constexpr bool sparse_gathers() { return KIND == K_AA_ODD || KIND == K_AB_PULL; }
@@ -144,15 +149,16 @@ struct SparseEmit {
    }
 };
 
-template <int Q, int KIND>
-__global__ void __launch_bounds__(kSparseAsyncWarps * 32, kSparseAsyncBlocks) sparse_async_kernel(
+template <int Q, int KIND, int FORCE>
+__global__ void __launch_bounds__(sparse_warps<Q>() * 32, sparse_blocks<Q>()) sparse_async_kernel(
    const KParams p, const int32_t* __restrict__ adj, uint32_t nf, uint32_t start, uint32_t count, uint32_t ntiles,
    const double* src, double* dst)
 {
    extern __shared__ __align__(16) unsigned long long sparse_smem[];
    const int lane = threadIdx.x & 31;
    const int warp = threadIdx.x >> 5;
-   const uint32_t nw = gridDim.x * kSparseAsyncWarps;
+   constexpr int kWarps = sparse_warps<Q>();
+   const uint32_t nw = gridDim.x * kWarps;
    wait_prior_grid();
    unsigned long long* mine = sparse_smem + (size_t)warp * kAsyncStages * Q * 32;
    const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(mine);
@@ -190,9 +196,9 @@ __global__ void __launch_bounds__(kSparseAsyncWarps * 32, kSparseAsyncBlocks) sp
    const bool fed = feed_on(ntiles, nw);
    TileFeed feed{0u, 0u, 1u, false};
    if (fed)
-      feed = feed_start(p.sched, 3u * nw, ntiles, blockIdx.x * kSparseAsyncWarps + warp, nw,
+      feed = feed_start(p.sched, 3u * nw, ntiles, blockIdx.x * kWarps + warp, nw,
                         Q == 19 ? kFeedGroups : 1u, lane);
-   uint32_t t = blockIdx.x * kSparseAsyncWarps + warp;
+   uint32_t t = blockIdx.x * kWarps + warp;
    if (t < ntiles) {
       uint32_t t1 = t + nw < ntiles ? t + nw : ntiles;
       uint32_t t2 = t + 2u * nw < ntiles ? t + 2u * nw : ntiles;
@@ -220,7 +226,7 @@ __global__ void __launch_bounds__(kSparseAsyncWarps * 32, kSparseAsyncBlocks) sp
                }
             }
             const SparseEmit<Q, KIND> emit{dst, nf, i, wl};
-            collide_f64x_shared_emit<Q>(mine + stage * Q * 32 + lane, p, emit);
+            collide_f64x_shared_emit<Q, FORCE>(mine + stage * Q * 32 + lane, p, emit);
          }
          if (t1 >= ntiles) break;
          t = t1;
@@ -232,8 +238,8 @@ __global__ void __launch_bounds__(kSparseAsyncWarps * 32, kSparseAsyncBlocks) sp
    if (fed) feed_done(p.sched);
 }
 
-template <int Q, int KIND>
-cudaError_t launch_sparse_async(const KParams& p, const int32_t* adj, int64_t nfluid, int64_t start, int64_t count,
+template <int Q, int KIND, int FORCE>
+cudaError_t launch_sparse_async_form(const KParams& p, const int32_t* adj, int64_t nfluid, int64_t start, int64_t count,
                                 const double* src, double* dst, cudaStream_t stream)
 {
    // persistent grid per device ordinal, set once (any thread computes the same value)
@@ -242,26 +248,38 @@ cudaError_t launch_sparse_async(const KParams& p, const int32_t* adj, int64_t nf
    cudaError_t e = cudaGetDevice(&dev);
    if (e != cudaSuccess) return e;
    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-   auto kern = sparse_async_kernel<Q, KIND>;
-   constexpr size_t smem = (size_t)kSparseAsyncWarps * kAsyncStages * Q * 32 * sizeof(unsigned long long);
+   constexpr int kWarps = sparse_warps<Q>(), kBlocks = sparse_blocks<Q>();
+   auto kern = sparse_async_kernel<Q, KIND, FORCE>;
+   constexpr size_t smem = (size_t)kWarps * kAsyncStages * Q * 32 * sizeof(unsigned long long);
    int cached = grid_of_device[dev].load(std::memory_order_relaxed);
    if (cached == 0) {
       e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
+      e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, carveout_percent(kBlocks, smem));
+      if (e != cudaSuccess) return e;
       int per_sm = 0, nsm = 0;
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSparseAsyncWarps * 32, smem);
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kWarps * 32, smem);
       if (e != cudaSuccess) return e;
       e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
       if (e != cudaSuccess) return e;
       if (per_sm < 1) return cudaErrorInvalidConfiguration;
-      cached = per_sm * nsm;
+      cached = (per_sm < kBlocks ? per_sm : kBlocks) * nsm;
       grid_of_device[dev].store(cached, std::memory_order_relaxed);
    }
    const uint32_t ntiles = (uint32_t)((count + 31) / 32);
-   const uint32_t need = (ntiles + kSparseAsyncWarps - 1) / kSparseAsyncWarps;
+   const uint32_t need = (ntiles + kWarps - 1) / kWarps;
    const unsigned grid = (unsigned)(need < (uint32_t)cached ? need : (uint32_t)cached);
-   return launch_overlapped(kern, dim3(grid), dim3(kSparseAsyncWarps * 32), smem, stream, p, adj, (uint32_t)nfluid,
+   return launch_overlapped(kern, dim3(grid), dim3(kWarps * 32), smem, stream, p, adj, (uint32_t)nfluid,
                             (uint32_t)start, (uint32_t)count, ntiles, src, dst);
+}
+
+template <int Q, int KIND>
+cudaError_t launch_sparse_async(const KParams& p, const int32_t* adj, int64_t nfluid, int64_t start, int64_t count,
+                                const double* src, double* dst, cudaStream_t stream)
+{
+   if (p.forced == 0) return launch_sparse_async_form<Q, KIND, 0>(p, adj, nfluid, start, count, src, dst, stream);
+   if (p.forced == 3) return launch_sparse_async_form<Q, KIND, 3>(p, adj, nfluid, start, count, src, dst, stream);
+   return launch_sparse_async_form<Q, KIND, kForceOther>(p, adj, nfluid, start, count, src, dst, stream);
 }
 
 template <int Q, int AR>

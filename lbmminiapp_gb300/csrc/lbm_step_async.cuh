@@ -25,20 +25,35 @@
 
 namespace lbm {
 
-// Warps per block and blocks per SM, measured on GB300: D3Q19 steps run best
-// with 8-warp blocks, two per SM (128 registers), D3Q27 steps with 4-warp
-// blocks, three per SM (at most 170 registers; at 128 they spill and run
-// 15-20 % slower).
-template <int Q, int KIND>
-constexpr int async_warps() { return Q == 19 ? 8 : 4; }
-template <int Q, int KIND>
-constexpr int async_min_blocks() { return async_warps<Q, KIND>() == 8 ? 2 : 3; }
+// Warps per block and blocks per SM.  What limits them is the L1 that the
+// shared memory leaves: every 8-byte cp.async passes through it, and its lines
+// bound the copies in flight.  At 256x128x128, with the blocks' shared memory
+// in the smallest carve-out that holds it (164 KB, 92 KB of L1), in the next
+// (196 KB) or in the largest (228 KB, 28 KB of L1):
+//   D3Q19 AA even / odd step   197 / 211 us,  -,               246 / 293 us
+//   D3Q27 AA even / odd step   283 / 342 us,  295 / 356 us,    362 / 438 us
+//   D3Q27 AB push / pull step  302 / 309 us,  316 / 305 us,    375 / 395 us
+// So D3Q19 runs 16 warps in two blocks (128 registers), D3Q27 12 warps in one
+// (168 registers; as three blocks the 1 KB that each reserves would take them
+// over 164 KB, and 16 warps need 228 KB), and the launch asks for the carve-out.
+template <int Q>
+constexpr int async_warps() { return Q == 19 ? 8 : 12; }
+template <int Q>
+constexpr int async_min_blocks() { return Q == 19 ? 2 : 1; }
 constexpr int kAsyncStages = 2;
+constexpr int kBlockReserve = 1024;          // shared memory the system takes per block
+constexpr int kMaxSharedPerSM = 228 * 1024;
 
-template <int Q, int KIND>
+// The smallest shared-memory carve-out (percent) that holds `blocks` blocks.
+constexpr int carveout_percent(int blocks, size_t smem)
+{
+   return (int)((blocks * (smem + kBlockReserve) * 100 + kMaxSharedPerSM - 1) / kMaxSharedPerSM);
+}
+
+template <int Q>
 constexpr size_t async_smem_bytes()
 {
-   return (size_t)async_warps<Q, KIND>() * kAsyncStages * Q * 32 * sizeof(unsigned long long);
+   return (size_t)async_warps<Q>() * kAsyncStages * Q * 32 * sizeof(unsigned long long);
 }
 
 // Tiles of 32 cells: tile t covers x in [32 (t mod ntx), +32) of row t / ntx,
@@ -108,27 +123,46 @@ __device__ __forceinline__ uint32_t tile_link(const KParams& p, const AsyncGeom&
 
 // lk: the tile's link words, loaded one tile ahead so the load's latency
 // hides behind a collision.
-// RAGGED: nx is not a multiple of 32, so some lanes fall past their row.
+// RAGGED: nx is not a multiple of 32, so some lanes fall past their row (with
+// LINKS their link word says so, and RAGGED is not looked at).
 template <bool LINKS, bool RAGGED>
 __device__ __forceinline__ void tile_lane(const KParams& p, const AsyncGeom& ag, uint32_t t, int lane, uint32_t lk,
                                           TileLane& tl)
 {
    const bool inside = tile_cell(p, ag, t, lane, tl.ci);
-   tl.active = RAGGED ? inside : true;
    tl.lk = LINKS ? lk : 0u;
-   if (LINKS) tl.active = tl.active && !(lk & kSolidBit);
+   tl.active = LINKS ? !(lk & kSolidBit) : (RAGGED ? inside : true);
 }
 
-template <int Q, int KIND, bool LINKS, bool RAGGED>
-__device__ __forceinline__ void async_issue(const PlanePtrs& pp, const TileLane& tl, int lane, uint32_t sbuf)
+// Whether any cell of the tile has a blocked neighbour (warp-uniform; every
+// lane calls it).  A tile without one runs its neighbour reads and writes
+// without the bounce-back selects, about six instructions per direction: on the
+// 256x128x128 channel the D3Q27 push step 336 -> 322 us, pull 332 -> 324 us, the
+// D3Q19 pull step 221 -> 216 us (with four-warp blocks).
+__device__ __forceinline__ bool tile_linked(uint32_t lk)
 {
-   if ((LINKS || RAGGED) && !tl.active) return;
+   return __any_sync(0xFFFFFFFFu, (lk & ~kSolidBit) != 0u);
+}
+
+template <int Q, int KIND, bool LINKS>
+__device__ __forceinline__ void async_issue_cell(const PlanePtrs& pp, const TileLane& tl, int lane, uint32_t sbuf)
+{
    const uint32_t c = (uint32_t)tl.ci.c;
 #pragma unroll
    for (int s = 0; s < Q; s++) {
       const Access a = read_access<Q, KIND, LINKS>(tl.ci, tl.lk, s);
       cp_async8(sbuf + (uint32_t)(s * 32 + lane) * 8u, pp.src[a.slot] + (c + (uint32_t)a.off));
    }
+}
+
+template <int Q, int KIND, bool LINKS, bool RAGGED>
+__device__ __forceinline__ void async_issue(const PlanePtrs& pp, const TileLane& tl, int lane, uint32_t sbuf)
+{
+   constexpr bool kGathers = KIND == K_AA_ODD || KIND == K_AB_PULL;
+   const bool linked = LINKS && kGathers && tile_linked(tl.lk);
+   if ((LINKS || RAGGED) && !tl.active) return;
+   if (LINKS && kGathers && linked) async_issue_cell<Q, KIND, LINKS>(pp, tl, lane, sbuf);
+   else async_issue_cell<Q, KIND, false>(pp, tl, lane, sbuf);
 }
 
 // Stores each output straight to its target slot.  AA stays race-free with
@@ -144,22 +178,16 @@ struct StoreEmit {
       const Access a = write_access<Q, KIND, LINKS>(ci, lk, s);
       pp.dst[a.slot][(uint32_t)ci.c + (uint32_t)a.off] = v;
    }
-   // A non-rest direction s known at run time, with o = opp(s) and c_s.
-   __device__ __forceinline__ void put(int s, int o, int cx, int cy, int cz, uint64_t v) const
-   {
-      const Access a = write_access_rt<KIND, LINKS>(ci, lk, s, o, cx, cy, cz);
-      pp.dst[a.slot][(uint32_t)ci.c + (uint32_t)a.off] = v;
-   }
 };
 
-template <int Q, int KIND, bool LINKS, bool RAGGED>
-__global__ void __launch_bounds__(async_warps<Q, KIND>() * 32, async_min_blocks<Q, KIND>()) step_async_kernel(const KParams p, const AsyncGeom ag,
+template <int Q, int KIND, bool LINKS, bool RAGGED, int FORCE>
+__global__ void __launch_bounds__(async_warps<Q>() * 32, async_min_blocks<Q>()) step_async_kernel(const KParams p, const AsyncGeom ag,
                                                                       const PlanePtrs pp)
 {
    extern __shared__ __align__(16) unsigned long long async_smem[];
    const int lane = threadIdx.x & 31;
    const int warp = threadIdx.x >> 5;
-   constexpr int kWarps = async_warps<Q, KIND>();
+   constexpr int kWarps = async_warps<Q>();
    const uint32_t nw = gridDim.x * kWarps;
    const uint32_t ntiles = ag.ntiles;
    wait_prior_grid();
@@ -191,16 +219,20 @@ __global__ void __launch_bounds__(async_warps<Q, KIND>() * 32, async_min_blocks<
          }
          cp_async_commit();
          cp_async_wait_prev();
+         // each output is stored as the collision makes it, and the update
+         // re-reads its inputs from shared memory: neither the Q input nor the
+         // Q output patterns stay in registers
+         constexpr bool kScatters = KIND == K_AA_ODD || KIND == K_AB_PUSH;
+         const unsigned long long* in = mine + stage * Q * 32 + lane;
+         const bool linked = LINKS && kScatters && tile_linked(cur.lk);
          if (!(LINKS || RAGGED) || cur.active) {
-            // each output is stored as the collision makes it, and the update
-            // re-reads its inputs from shared memory: neither the Q input nor the
-            // Q output patterns stay in registers
-            // D3Q27 AB pull (stores to the cell's own slots) runs the pair-class
-            // loops: 9.69 -> 9.96 GLUPS on the 256x128x128 channel.  Where the
-            // stores go to neighbours (AB push: 9.92 -> 9.12) each store's
-            // offset would cost more than the smaller code saves.
-            StoreEmit<Q, KIND, LINKS> emit{pp, cur.ci, cur.lk};
-            collide_f64x_shared_emit<Q, Q == 27 && KIND == K_AB_PULL>(mine + stage * Q * 32 + lane, p, emit);
+            if (LINKS && kScatters && linked) {
+               StoreEmit<Q, KIND, LINKS> emit{pp, cur.ci, cur.lk};
+               collide_f64x_shared_emit<Q, FORCE>(in, p, emit);
+            } else {
+               StoreEmit<Q, KIND, false> emit{pp, cur.ci, 0u};
+               collide_f64x_shared_emit<Q, FORCE>(in, p, emit);
+            }
          }
          if (t1 >= ntiles) break;
          t = t1;
@@ -225,8 +257,8 @@ inline AsyncGeom async_geom(int nx, int ny, int nz)
 
 // Persistent grid: as many blocks as fit on the device at once (queried once
 // per device and kernel; the shared-memory opt-in is set at the same time).
-template <int Q, int KIND, bool LINKS, bool RAGGED>
-cudaError_t launch_async(const KParams& p, const AsyncGeom& ag, const void* src, void* dst, cudaStream_t stream)
+template <int Q, int KIND, bool LINKS, bool RAGGED, int FORCE>
+cudaError_t launch_async_form(const KParams& p, const AsyncGeom& ag, const void* src, void* dst, cudaStream_t stream)
 {
    // Persistent grid size per device ordinal, set once (the value is the same
    // whichever thread computes it first).
@@ -235,12 +267,15 @@ cudaError_t launch_async(const KParams& p, const AsyncGeom& ag, const void* src,
    cudaError_t e = cudaGetDevice(&dev);
    if (e != cudaSuccess) return e;
    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-   auto kern = step_async_kernel<Q, KIND, LINKS, RAGGED>;
-   constexpr int kWarps = async_warps<Q, KIND>();
-   constexpr size_t smem = async_smem_bytes<Q, KIND>();
+   auto kern = step_async_kernel<Q, KIND, LINKS, RAGGED, FORCE>;
+   constexpr int kWarps = async_warps<Q>();
+   constexpr size_t smem = async_smem_bytes<Q>();
    int cached = grid_of_device[dev].load(std::memory_order_relaxed);
    if (cached == 0) {
       e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+      e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
+                               carveout_percent(async_min_blocks<Q>(), smem));
       if (e != cudaSuccess) return e;
       int per_sm = 0, nsm = 0;
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kWarps * 32, smem);
@@ -248,7 +283,8 @@ cudaError_t launch_async(const KParams& p, const AsyncGeom& ag, const void* src,
       e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
       if (e != cudaSuccess) return e;
       if (per_sm < 1) return cudaErrorInvalidConfiguration;
-      cached = per_sm * nsm;
+      // no more than the carve-out is meant for
+      cached = (per_sm < async_min_blocks<Q>() ? per_sm : async_min_blocks<Q>()) * nsm;
       grid_of_device[dev].store(cached, std::memory_order_relaxed);
    }
    const uint32_t need = (ag.ntiles + kWarps - 1) / kWarps;
@@ -261,5 +297,36 @@ cudaError_t launch_async(const KParams& p, const AsyncGeom& ag, const void* src,
    }
    return launch_overlapped(kern, dim3(grid), dim3(kWarps * 32), smem, stream, p, ag, pp);
 }
+
+// links: the grid has link words.  Kernels exist for no force and the velocity
+// shift with full and ragged rows; the other forcing forms run the ragged form
+// for every row length.
+template <int Q, int KIND>
+cudaError_t launch_async_kind(bool links, const KParams& p, const AsyncGeom& ag, const void* src, void* dst,
+                              cudaStream_t stream)
+{
+   const bool ragged = p.nx % 32 != 0;
+   if (p.forced == 0) {
+      if (links) return launch_async_form<Q, KIND, true, false, 0>(p, ag, src, dst, stream);
+      return ragged ? launch_async_form<Q, KIND, false, true, 0>(p, ag, src, dst, stream)
+                    : launch_async_form<Q, KIND, false, false, 0>(p, ag, src, dst, stream);
+   }
+   if (p.forced == 3) {
+      if (links) return launch_async_form<Q, KIND, true, false, 3>(p, ag, src, dst, stream);
+      return ragged ? launch_async_form<Q, KIND, false, true, 3>(p, ag, src, dst, stream)
+                    : launch_async_form<Q, KIND, false, false, 3>(p, ag, src, dst, stream);
+   }
+   return links ? launch_async_form<Q, KIND, true, false, kForceOther>(p, ag, src, dst, stream)
+                : launch_async_form<Q, KIND, false, true, kForceOther>(p, ag, src, dst, stream);
+}
+
+// launch_async_kind for a kind known at run time; instantiated in
+// lbm_step_q*_aa.cu and lbm_step_q*_ab.cu, so the library builds in parallel.
+template <int Q>
+cudaError_t launch_async_aa(int kind, bool links, const KParams& p, const AsyncGeom& ag, const void* src, void* dst,
+                            cudaStream_t stream);
+template <int Q>
+cudaError_t launch_async_ab(int kind, bool links, const KParams& p, const AsyncGeom& ag, const void* src, void* dst,
+                            cudaStream_t stream);
 
 }  // namespace lbm
