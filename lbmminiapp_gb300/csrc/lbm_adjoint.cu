@@ -26,290 +26,303 @@
 // Loss terms at step t (weight tw, spatial weights W):
 //   velocity:  L_t = tw sum_x W(x) . u(x)        dL/df_k = tw W.(c_k - u)/rho, dL/dF = tw W/(2 rho)
 //   energy:    L_t = tw sum_x W_0(x) rho|u|^2/2   dL/df_k = tw W_0 (u.c_k - |u|^2/2), dL/dF = tw W_0 u/2
-// adjoint_step_kernel works in FP64.  adjoint_step_f32_kernel is the same
-// step with lam and the arithmetic in FP32, written on the deviations
-// g_s = f_s - w_s (the shifted storage formats hold exactly these), so that
-// f_opp(s) - C_s = g_opp(s) - (C_s - w_s) has no cancellation against w; its
-// gradients are still accumulated in FP64.  f^t may be stored in any storage
-// format.
+// The sums over s need mu only through the weighted moments
+//   m0 = sum w mu, m1 = sum w mu c, m2 = sum w mu c c^T
+// (with nu = (1 - sig) mu a common factor):
+//   T     = 3 m1 + 9 m2 u - 3 m0 u
+//   A_rho = (1 - sig) [omega ((1 + 3/2 uu) m0 - 9/2 u.m2.u) + (1 - omega/2)/rho (3 F.u m0 - 9 F.m2.u)]
+//   A_j   = (1 - sig) [omega T + (1 - omega/2)/rho (9 m2 F - 3 m0 F)]
+//   sum_s nu_s (1 - omega/2) dfd_s/dF = (1 - sig) (1 - omega/2) T
+//   sum_s mu_s C_s from m0, m1, m2 and sum mu_s f_s
+// and opposite directions enter them by their sum and difference.  That is about
+// 265 operations per D3Q19 cell; direction by direction it was 1180, and the
+// FP64 form is bound by the FP64 pipe (76 cycles per instruction, warp and
+// sub-partition).  Everything is written on the deviations g_s = f_s - w_s (the
+// shifted storage formats hold exactly these), so that f_opp(s) - C_s has no
+// cancellation against w.
+//
+// One kernel for both adjoints: R = double, and R = float with lam and the
+// arithmetic in FP32.  The gradients are accumulated in FP64 either way; f^t may
+// be stored in any storage format.
 #include <cuda_runtime.h>
 
 #include "../../include/lbm_gb300.h"
 #include "lbm_adjoint.cuh"
 #include "lbm_aux.cuh"
+#include "lbm_moments.cuh"
+#include "lbm_step.cuh"
 
 namespace lbm {
 
-template <int Q, int ST>
-__global__ void __launch_bounds__(128) adjoint_step_kernel(AdjParams a)
-{
-   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-   int x, y, z;
-   if (!cell_xyz(a.g, c, x, y, z)) return;
-   const uint32_t lk = a.links ? a.links[c] : 0u;
-   if (lk & kSolidBit) {
-#pragma unroll
-      for (int s = 0; s < Q; s++) a.lam[(int64_t)s * a.g.plane + c] = 0.0;
-      return;
-   }
-   double f[Q];
-#pragma unroll
-   for (int s = 0; s < Q; s++) f[s] = load_pop<ST>(a.state, (int64_t)s * a.g.plane + c, lat_w(Q, s));
-   double F[3] = {a.F[0], a.F[1], a.F[2]};
-   if (a.force_field) {
-      F[0] += a.force_field[c];
-      F[1] += a.force_field[a.g.plane + c];
-      F[2] += a.force_field[2 * a.g.plane + c];
-   }
-   const double sig = a.porosity ? a.porosity[c] : 0.0;
-   double rho = 0.0, j[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-   for (int s = 0; s < Q; s++) {
-      rho += f[s];
-      j[0] += f[s] * lat_c(Q, s, 0);
-      j[1] += f[s] * lat_c(Q, s, 1);
-      j[2] += f[s] * lat_c(Q, s, 2);
-   }
-   const double ir = 1.0 / rho;
-   double u[3];
-#pragma unroll
-   for (int d = 0; d < 3; d++) {
-      j[d] += 0.5 * F[d];
-      u[d] = j[d] * ir;
-   }
-   const double uu = u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
-   const double Fu = F[0] * u[0] + F[1] * u[1] + F[2] * u[2];
-   const double om = a.omega, om1 = 1.0 - om, om2 = 1.0 - 0.5 * om;
-
-   double lam[Q];
-#pragma unroll
-   for (int s = 0; s < Q; s++) lam[s] = 0.0;
-   double gF[3] = {0.0, 0.0, 0.0};
-   double gsig = 0.0;
-
-   if (a.collide) {
-      // mu: streaming transposed
-      double mu[Q];
-#pragma unroll
-      for (int s = 0; s < Q; s++) {
-         if (s == lat_rest(Q)) {
-            mu[s] = a.lam_next[(int64_t)s * a.g.plane + c];
-         } else if ((lk >> s) & 1u) {
-            mu[s] = a.lam_next[(int64_t)lat_opp(Q, s) * a.g.plane + c];
-         } else {
-            const int64_t n = nbr_cell(a.g, x, y, z, lat_c(Q, s, 0), lat_c(Q, s, 1), lat_c(Q, s, 2));
-            mu[s] = a.lam_next[(int64_t)s * a.g.plane + n];
-         }
-      }
-      double Arho = 0.0, Aj[3] = {0.0, 0.0, 0.0}, GF[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-      for (int s = 0; s < Q; s++) {
-         const double c0 = lat_c(Q, s, 0), c1 = lat_c(Q, s, 1), c2 = lat_c(Q, s, 2);
-         const double w = lat_w(Q, s);
-         const double cu = c0 * u[0] + c1 * u[1] + c2 * u[2];
-         const double cF = c0 * F[0] + c1 * F[1] + c2 * F[2];
-         const double cj = c0 * j[0] + c1 * j[1] + c2 * j[2];
-         // C_s for the porosity gradient
-         const double eq = w * (rho + 3.0 * cj + 4.5 * cj * cu - 1.5 * uu * rho);
-         const double fd = w * (3.0 * cF - 3.0 * Fu + 9.0 * cu * cF);
-         const double Cs = om1 * f[s] + om * eq + om2 * fd;
-         gsig += mu[s] * (f[lat_opp(Q, s)] - Cs);
-         const double nu = (1.0 - sig) * mu[s];
-         lam[s] += om1 * nu;
-         lam[lat_opp(Q, s)] += sig * mu[s];
-         // d/drho and d/dj of omega eq + om2 fd
-         const double deq_drho = w * (1.0 - 4.5 * cu * cu + 1.5 * uu);
-         const double dfd_drho = w * (3.0 * Fu - 9.0 * cu * cF) * ir;
-         Arho += nu * (om * deq_drho + om2 * dfd_drho);
-         const double ce = 3.0 + 9.0 * cu;      // coefficient of c in deq/dj (over w)
-         const double cfd = 9.0 * cF * ir;      // coefficient of c in dfd/dj (over w)
-         const double kc = nu * w * (om * ce + om2 * cfd);
-         Aj[0] += kc * c0 - nu * w * (om * 3.0 * u[0] + om2 * 3.0 * F[0] * ir);
-         Aj[1] += kc * c1 - nu * w * (om * 3.0 * u[1] + om2 * 3.0 * F[1] * ir);
-         Aj[2] += kc * c2 - nu * w * (om * 3.0 * u[2] + om2 * 3.0 * F[2] * ir);
-         // explicit dfd/dF at fixed j: w (3 c - 3 u + 9 (c.u) c)
-         const double kf = nu * om2 * w;
-         GF[0] += kf * (3.0 * c0 - 3.0 * u[0] + 9.0 * cu * c0);
-         GF[1] += kf * (3.0 * c1 - 3.0 * u[1] + 9.0 * cu * c1);
-         GF[2] += kf * (3.0 * c2 - 3.0 * u[2] + 9.0 * cu * c2);
-      }
-#pragma unroll
-      for (int s = 0; s < Q; s++)
-         lam[s] += Arho + Aj[0] * lat_c(Q, s, 0) + Aj[1] * lat_c(Q, s, 1) + Aj[2] * lat_c(Q, s, 2);
-#pragma unroll
-      for (int d = 0; d < 3; d++) gF[d] = GF[d] + 0.5 * Aj[d];
-   }
-
-   // loss at this step
-   if (a.loss_kind == LBM_LOSS_VELOCITY && a.loss_weight) {
-      const double W[3] = {a.loss_weight[c], a.loss_weight[a.g.plane + c], a.loss_weight[2 * a.g.plane + c]};
-      const double tw = a.time_weight;
-      const double Wu = W[0] * u[0] + W[1] * u[1] + W[2] * u[2];
-#pragma unroll
-      for (int s = 0; s < Q; s++) {
-         const double Wc = W[0] * lat_c(Q, s, 0) + W[1] * lat_c(Q, s, 1) + W[2] * lat_c(Q, s, 2);
-         lam[s] += tw * (Wc - Wu) * ir;
-      }
-#pragma unroll
-      for (int d = 0; d < 3; d++) gF[d] += tw * W[d] * 0.5 * ir;
-   } else if (a.loss_kind == LBM_LOSS_ENERGY && a.loss_weight) {
-      const double tw = a.time_weight * a.loss_weight[c];
-#pragma unroll
-      for (int s = 0; s < Q; s++) {
-         const double uc = u[0] * lat_c(Q, s, 0) + u[1] * lat_c(Q, s, 1) + u[2] * lat_c(Q, s, 2);
-         lam[s] += tw * (uc - 0.5 * uu);
-      }
-#pragma unroll
-      for (int d = 0; d < 3; d++) gF[d] += tw * 0.5 * u[d];
-   }
-
-#pragma unroll
-   for (int s = 0; s < Q; s++) a.lam[(int64_t)s * a.g.plane + c] = lam[s];
-   if (a.grad_force) {
-#pragma unroll
-      for (int d = 0; d < 3; d++) a.grad_force[(int64_t)d * a.g.plane + c] += gF[d];
-   }
-   if (a.grad_porosity) a.grad_porosity[c] += gsig;
-}
-
-// FP32 deviation g = f - w of a stored population.
-template <int ST>
-__device__ __forceinline__ float load_dev(const void* buf, int64_t idx, double w)
+// Deviation g = f - w of a stored population.
+template <int ST, typename R>
+__device__ __forceinline__ R load_dev(const void* buf, int64_t idx, double w)
 {
    if constexpr (ST == ST_F64) {
-      return (float)(static_cast<const double*>(buf)[idx] - w);
+      return (R)(static_cast<const double*>(buf)[idx] - w);
    } else {
-      return load_shifted(static_cast<const typename Store<ST>::T*>(buf) + idx);
+      return (R)load_shifted(static_cast<const typename Store<ST>::T*>(buf) + idx);
    }
 }
 
-template <int Q, int ST>
-__global__ void __launch_bounds__(256) adjoint_step_f32_kernel(AdjParams a)
+// The adjoint buffers and the launch constants in the kernel's arithmetic.
+template <typename R> struct AdjBuffers;
+template <> struct AdjBuffers<double> {
+   __device__ static const double* next(const AdjParams& a) { return a.lam_next; }
+   __device__ static double* out(const AdjParams& a) { return a.lam; }
+   __device__ static const AdjConsts<double>& k(const AdjParams& a) { return a.k; }
+};
+template <> struct AdjBuffers<float> {
+   __device__ static const float* next(const AdjParams& a) { return a.lam_next_f; }
+   __device__ static float* out(const AdjParams& a) { return a.lam_f; }
+   __device__ static const AdjConsts<float>& k(const AdjParams& a) { return a.kf; }
+};
+
+// One cell's position and neighbour offsets (32-bit: fewer than 2^31 cells).
+__device__ __forceinline__ bool adj_cell(const GridDims& g, CellIndex& ci)
 {
-   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-   int x, y, z;
-   if (!cell_xyz(a.g, c, x, y, z)) return;
+   const int x = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+   if (x >= g.nx) return false;
+   const int y = (int)blockIdx.y, z = (int)blockIdx.z;
+   ci.c = ((int64_t)z * g.ny + y) * g.nx + x;
+   ci.dxm = (x == 0) ? g.nx - 1 : -1;
+   ci.dxp = (x == g.nx - 1) ? -(g.nx - 1) : 1;
+   ci.dym = (y == 0) ? (g.ny - 1) * g.nx : -g.nx;
+   ci.dyp = (y == g.ny - 1) ? -(g.ny - 1) * g.nx : g.nx;
+   const int nxy = g.nx * g.ny;
+   ci.dzm = (z == 0) ? (g.nz - 1) * nxy : -nxy;
+   ci.dzp = (z == g.nz - 1) ? -(g.nz - 1) * nxy : nxy;
+   return true;
+}
+
+template <int Q, int ST, typename R>
+__global__ void __launch_bounds__(128) adjoint_step_kernel(const AdjParams a)
+{
+   CellIndex ci;
+   if (!adj_cell(a.g, ci)) return;
+   const int64_t c = ci.c, plane = a.g.plane;
    const uint32_t lk = a.links ? a.links[c] : 0u;
+   R* lam = AdjBuffers<R>::out(a);
+   const AdjConsts<R>& K = AdjBuffers<R>::k(a);
    if (lk & kSolidBit) {
 #pragma unroll
-      for (int s = 0; s < Q; s++) a.lam_f[(int64_t)s * a.g.plane + c] = 0.0f;
+      for (int s = 0; s < Q; s++) lam[(int64_t)s * plane + c] = R(0);
       return;
    }
-   float g[Q];
+   constexpr int NP = (Q - 1) / 2, RD = lat_rest(Q);
+   const R* next = AdjBuffers<R>::next(a);
+   // mu (streaming transposed): per pair its sum and difference
+   R p[NP], d[NP], mur = R(0);
 #pragma unroll
-   for (int s = 0; s < Q; s++) g[s] = load_dev<ST>(a.state, (int64_t)s * a.g.plane + c, lat_w(Q, s));
-   float F[3] = {(float)a.F[0], (float)a.F[1], (float)a.F[2]};
-   if (a.force_field) {
-      F[0] = (float)(a.F[0] + a.force_field[c]);
-      F[1] = (float)(a.F[1] + a.force_field[a.g.plane + c]);
-      F[2] = (float)(a.F[2] + a.force_field[2 * a.g.plane + c]);
+   for (int q = 0; q < NP; q++) {
+      p[q] = d[q] = R(0);
+      if (a.collide) {
+         const int s = pair_dir(Q, q), o = lat_opp(Q, s);
+         const bool bs = (lk >> s) & 1u, bo = (lk >> o) & 1u;
+         const int off = nbr_off(ci, lat_c(Q, s, 0), lat_c(Q, s, 1), lat_c(Q, s, 2));
+         const int ofo = nbr_off(ci, lat_c(Q, o, 0), lat_c(Q, o, 1), lat_c(Q, o, 2));
+         const R ms = next[(int64_t)(bs ? o : s) * plane + (c + (bs ? 0 : off))];
+         const R mo = next[(int64_t)(bo ? s : o) * plane + (c + (bo ? 0 : ofo))];
+         p[q] = ms + mo;
+         d[q] = ms - mo;
+      }
    }
-   const float sig = a.porosity ? (float)a.porosity[c] : 0.0f;
-   float drho = 0.0f, j[3] = {0.0f, 0.0f, 0.0f};
-#pragma unroll
-   for (int s = 0; s < Q; s++) {
-      drho += g[s];
-      j[0] += g[s] * (float)lat_c(Q, s, 0);
-      j[1] += g[s] * (float)lat_c(Q, s, 1);
-      j[2] += g[s] * (float)lat_c(Q, s, 2);
-   }
-   const float rho = 1.0f + drho;
-   const float ir = 1.0f / rho;
-   float u[3];
-#pragma unroll
-   for (int d = 0; d < 3; d++) {
-      j[d] += 0.5f * F[d];
-      u[d] = j[d] * ir;
-   }
-   const float uu = u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
-   const float Fu = F[0] * u[0] + F[1] * u[1] + F[2] * u[2];
-   const float om = (float)a.omega, om1 = (float)(1.0 - a.omega), om2 = (float)(1.0 - 0.5 * a.omega);
+   if (a.collide) mur = next[(int64_t)RD * plane + c];
 
-   float lam[Q];
+   // drho, j and the products with mu of the porosity gradient, in one pass over f:
+   // dot1 = sum over pairs (f_s - f_o)(mu_s - mu_o), dot0 = sum of (g_s + g_o)(mu_s + mu_o)
+   const R gr = load_dev<ST, R>(a.state, (int64_t)RD * plane + c, lat_w(Q, RD));
+   R drho = gr, j[3] = {R(0), R(0), R(0)}, dot1 = R(0), dot0 = R(0);
+   R m0 = (R)lat_w(Q, RD) * mur, m1[3] = {R(0), R(0), R(0)}, md[3] = {R(0), R(0), R(0)}, mo_[3] = {R(0), R(0), R(0)};
+   // axes
+   {
+      R ps = R(0);
 #pragma unroll
-   for (int s = 0; s < Q; s++) lam[s] = 0.0f;
-   float gF[3] = {0.0f, 0.0f, 0.0f};
-   float gsig = 0.0f;
-
-   if (a.collide) {
-      float mu[Q];
-#pragma unroll
-      for (int s = 0; s < Q; s++) {
-         if (s == lat_rest(Q)) {
-            mu[s] = a.lam_next_f[(int64_t)s * a.g.plane + c];
-         } else if ((lk >> s) & 1u) {
-            mu[s] = a.lam_next_f[(int64_t)lat_opp(Q, s) * a.g.plane + c];
+      for (int k = 0; k < 3; k++) {
+         const int s = 2 * k, o = 2 * k + 1;
+         const double w = lat_w(Q, s);
+         R S, D;
+         if constexpr (ST == ST_F64 && sizeof(R) == 8) {
+            const double fs = static_cast<const double*>(a.state)[(int64_t)s * plane + c];
+            const double fo = static_cast<const double*>(a.state)[(int64_t)o * plane + c];
+            S = (fs + fo) - 2.0 * w;
+            D = fs - fo;
          } else {
-            const int64_t n = nbr_cell(a.g, x, y, z, lat_c(Q, s, 0), lat_c(Q, s, 1), lat_c(Q, s, 2));
-            mu[s] = a.lam_next_f[(int64_t)s * a.g.plane + n];
+            const R gs = load_dev<ST, R>(a.state, (int64_t)s * plane + c, w);
+            const R go = load_dev<ST, R>(a.state, (int64_t)o * plane + c, w);
+            S = gs + go;
+            D = gs - go;
          }
+         drho += S;
+         j[k] = D;
+         dot1 += D * d[k];
+         dot0 += S * p[k];
+         ps += p[k];
+         m1[k] = (R)w * d[k];
+         md[k] = (R)w * p[k];
       }
-      float Arho = 0.0f, Aj[3] = {0.0f, 0.0f, 0.0f}, GF[3] = {0.0f, 0.0f, 0.0f};
+      m0 += (R)lat_w(Q, 0) * ps;
+   }
+   // planes: pairs c = e_a + e_b (q1) and e_a - e_b (q2)
+   {
+      constexpr double w = lat_w(Q, 6);
+      R ps = R(0);
 #pragma unroll
-      for (int s = 0; s < Q; s++) {
-         const float c0 = (float)lat_c(Q, s, 0), c1 = (float)lat_c(Q, s, 1), c2 = (float)lat_c(Q, s, 2);
-         const float w = (float)lat_w(Q, s);
-         const float cu = c0 * u[0] + c1 * u[1] + c2 * u[2];
-         const float cF = c0 * F[0] + c1 * F[1] + c2 * F[2];
-         const float cj = c0 * j[0] + c1 * j[1] + c2 * j[2];
-         // C_s - w_s for the porosity gradient
-         const float eqd = w * (drho + 3.0f * cj + 4.5f * cj * cu - 1.5f * uu * rho);
-         const float fd = w * (3.0f * cF - 3.0f * Fu + 9.0f * cu * cF);
-         const float Cd = om1 * g[s] + om * eqd + om2 * fd;
-         gsig += mu[s] * (g[lat_opp(Q, s)] - Cd);
-         const float nu = (1.0f - sig) * mu[s];
-         lam[s] += om1 * nu;
-         lam[lat_opp(Q, s)] += sig * mu[s];
-         const float deq_drho = w * (1.0f - 4.5f * cu * cu + 1.5f * uu);
-         const float dfd_drho = w * (3.0f * Fu - 9.0f * cu * cF) * ir;
-         Arho += nu * (om * deq_drho + om2 * dfd_drho);
-         const float kc = nu * w * (om * (3.0f + 9.0f * cu) + om2 * 9.0f * cF * ir);
-         Aj[0] += kc * c0 - nu * w * (om * 3.0f * u[0] + om2 * 3.0f * F[0] * ir);
-         Aj[1] += kc * c1 - nu * w * (om * 3.0f * u[1] + om2 * 3.0f * F[1] * ir);
-         Aj[2] += kc * c2 - nu * w * (om * 3.0f * u[2] + om2 * 3.0f * F[2] * ir);
-         const float kf = nu * om2 * w;
-         GF[0] += kf * (3.0f * c0 - 3.0f * u[0] + 9.0f * cu * c0);
-         GF[1] += kf * (3.0f * c1 - 3.0f * u[1] + 9.0f * cu * c1);
-         GF[2] += kf * (3.0f * c2 - 3.0f * u[2] + 9.0f * cu * c2);
+      for (int k = 0; k < 3; k++) {
+         const int A = k < 2 ? 0 : 1, B = k == 0 ? 1 : 2;
+         const int q1 = 3 + 2 * k, q2 = q1 + 1;
+         R S[2], D[2];
+#pragma unroll
+         for (int h = 0; h < 2; h++) {
+            const int s = pair_dir(Q, q1 + h), o = lat_opp(Q, s);
+            if constexpr (ST == ST_F64 && sizeof(R) == 8) {
+               const double fs = static_cast<const double*>(a.state)[(int64_t)s * plane + c];
+               const double fo = static_cast<const double*>(a.state)[(int64_t)o * plane + c];
+               S[h] = (fs + fo) - 2.0 * w;
+               D[h] = fs - fo;
+            } else {
+               const R gs = load_dev<ST, R>(a.state, (int64_t)s * plane + c, w);
+               const R go = load_dev<ST, R>(a.state, (int64_t)o * plane + c, w);
+               S[h] = gs + go;
+               D[h] = gs - go;
+            }
+            drho += S[h];
+            dot1 += D[h] * d[q1 + h];
+            dot0 += S[h] * p[q1 + h];
+         }
+         j[A] += D[0] + D[1];
+         j[B] += D[0] - D[1];
+         const R pp = p[q1] + p[q2];
+         ps += pp;
+         m1[A] += (R)w * (d[q1] + d[q2]);
+         m1[B] += (R)w * (d[q1] - d[q2]);
+         md[A] += (R)w * pp;
+         md[B] += (R)w * pp;
+         mo_[k] = (R)w * (p[q1] - p[q2]);
       }
+      m0 += (R)w * ps;
+   }
+   // bodies: c = (1, +-1, +-1)
+   if constexpr (Q == 27) {
+      constexpr double w = lat_w(Q, 18);
 #pragma unroll
-      for (int s = 0; s < Q; s++)
-         lam[s] += Arho + Aj[0] * (float)lat_c(Q, s, 0) + Aj[1] * (float)lat_c(Q, s, 1) +
-                   Aj[2] * (float)lat_c(Q, s, 2);
-#pragma unroll
-      for (int d = 0; d < 3; d++) gF[d] = GF[d] + 0.5f * Aj[d];
+      for (int h = 0; h < 4; h++) {
+         const int q = 9 + h, s = pair_dir(Q, q), o = lat_opp(Q, s);
+         const R gs = load_dev<ST, R>(a.state, (int64_t)s * plane + c, w);
+         const R go = load_dev<ST, R>(a.state, (int64_t)o * plane + c, w);
+         const R S = gs + go, D = gs - go;
+         const R cy = (R)lat_c(Q, s, 1), cz = (R)lat_c(Q, s, 2);   // +-1
+         drho += S;
+         j[0] += D;
+         j[1] += cy * D;
+         j[2] += cz * D;
+         dot1 += D * d[q];
+         dot0 += S * p[q];
+         const R wd = (R)w * d[q], wp = (R)w * p[q];
+         m0 += wp;
+         m1[0] += wd;
+         m1[1] += cy * wd;
+         m1[2] += cz * wd;
+         md[0] += wp;
+         md[1] += wp;
+         md[2] += wp;
+         mo_[0] += cy * wp;
+         mo_[1] += cz * wp;
+         mo_[2] += (cy * cz) * wp;
+      }
    }
 
+   // force: (R)(F + field), the fields' FP32 copies where they hold that value
+   R F[3];
+#pragma unroll
+   for (int k = 0; k < 3; k++) {
+      if (sizeof(R) == 4 && a.force_field_f) F[k] = a.force_field_f[k * plane + c];
+      else F[k] = a.force_field ? (R)(a.F[k] + a.force_field[k * plane + c]) : K.F[k];
+   }
+   R sig = R(0);
+   if (sizeof(R) == 4 && a.porosity_f) sig = a.porosity_f[c];
+   else if (a.porosity) sig = (R)a.porosity[c];
+   const R rho = R(1) + drho;
+   const R ir = R(1) / rho;
+   R u[3];
+#pragma unroll
+   for (int k = 0; k < 3; k++) {
+      j[k] += R(0.5) * F[k];
+      u[k] = j[k] * ir;
+   }
+   const R uu = u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
+   const R Fu = F[0] * u[0] + F[1] * u[1] + F[2] * u[2];
+   const R om = K.om, om1 = K.om1, om2 = K.om2;
+
+   R even = R(0), odd[3] = {R(0), R(0), R(0)};   // lam_k = (1-omega) nu_k + sig mu_opp + even + odd . c_k
+   R gF[3] = {R(0), R(0), R(0)}, gsig = R(0);
+   const R keep = R(1) - sig;
+   if (a.collide) {
+      const R mu_u[3] = {md[0] * u[0] + mo_[0] * u[1] + mo_[1] * u[2], mo_[0] * u[0] + md[1] * u[1] + mo_[2] * u[2],
+                         mo_[1] * u[0] + mo_[2] * u[1] + md[2] * u[2]};
+      const R mu_F[3] = {md[0] * F[0] + mo_[0] * F[1] + mo_[1] * F[2], mo_[0] * F[0] + md[1] * F[1] + mo_[2] * F[2],
+                         mo_[1] * F[0] + mo_[2] * F[1] + md[2] * F[2]};
+      const R uMu = u[0] * mu_u[0] + u[1] * mu_u[1] + u[2] * mu_u[2];
+      const R FMu = F[0] * mu_u[0] + F[1] * mu_u[1] + F[2] * mu_u[2];
+      const R o2r = om2 * ir;
+      const R ffe = R(3) * Fu * m0 - R(9) * FMu;
+      even = keep * (om * ((R(1) + R(1.5) * uu) * m0 - R(4.5) * uMu) + o2r * ffe);
+      R jm = R(0), Fm = R(0);
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+         const R T = R(3) * (m1[k] + R(3) * mu_u[k] - m0 * u[k]);
+         odd[k] = keep * (om * T + o2r * (R(9) * mu_F[k] - R(3) * m0 * F[k]));
+         gF[k] = keep * (om2 * T) + R(0.5) * odd[k];
+         jm += m1[k] * j[k];
+         Fm += m1[k] * F[k];
+      }
+      // sum_s mu_s (f_opp(s) - C_s) = -dot1 + omega (sum mu g - sum mu (eq - w)) - om2 sum mu fd
+      const R mug = R(0.5) * (dot0 + dot1) + mur * gr;
+      const R mueq = (drho - R(1.5) * uu * rho) * m0 + R(3) * jm + R(4.5) * rho * uMu;
+      const R mufd = R(3) * Fm - ffe;
+      gsig = om * (mug - mueq) - dot1 - om2 * mufd;
+   }
+   // loss at this step
    if (a.loss_kind == LBM_LOSS_VELOCITY && a.loss_weight) {
-      const float tw = (float)a.time_weight;
-      const float W[3] = {(float)a.loss_weight[c], (float)a.loss_weight[a.g.plane + c],
-                          (float)a.loss_weight[2 * a.g.plane + c]};
-      const float Wu = W[0] * u[0] + W[1] * u[1] + W[2] * u[2];
+      const R W[3] = {(R)a.loss_weight[c], (R)a.loss_weight[plane + c], (R)a.loss_weight[2 * plane + c]};
+      const R tw = K.tw * ir;
+      even -= tw * (W[0] * u[0] + W[1] * u[1] + W[2] * u[2]);
 #pragma unroll
-      for (int s = 0; s < Q; s++) {
-         const float Wc = W[0] * (float)lat_c(Q, s, 0) + W[1] * (float)lat_c(Q, s, 1) + W[2] * (float)lat_c(Q, s, 2);
-         lam[s] += tw * (Wc - Wu) * ir;
+      for (int k = 0; k < 3; k++) {
+         odd[k] += tw * W[k];
+         gF[k] += R(0.5) * tw * W[k];
       }
-#pragma unroll
-      for (int d = 0; d < 3; d++) gF[d] += tw * W[d] * 0.5f * ir;
    } else if (a.loss_kind == LBM_LOSS_ENERGY && a.loss_weight) {
-      const float tw = (float)(a.time_weight * a.loss_weight[c]);
+      const R tw = (R)(a.time_weight * a.loss_weight[c]);
+      even -= R(0.5) * tw * uu;
 #pragma unroll
-      for (int s = 0; s < Q; s++) {
-         const float uc = u[0] * (float)lat_c(Q, s, 0) + u[1] * (float)lat_c(Q, s, 1) + u[2] * (float)lat_c(Q, s, 2);
-         lam[s] += tw * (uc - 0.5f * uu);
+      for (int k = 0; k < 3; k++) {
+         odd[k] += tw * u[k];
+         gF[k] += R(0.5) * tw * u[k];
       }
-#pragma unroll
-      for (int d = 0; d < 3; d++) gF[d] += tw * 0.5f * u[d];
    }
 
+   const R k1 = om1 * keep;
+   const R al = R(0.5) * (k1 + sig), be = R(0.5) * (k1 - sig);
+   lam[(int64_t)RD * plane + c] = (k1 + sig) * mur + even;
+   R op[3] = {odd[0] + odd[1], odd[0] + odd[2], odd[1] + odd[2]};
+   R om_[3] = {odd[0] - odd[1], odd[0] - odd[2], odd[1] - odd[2]};
 #pragma unroll
-   for (int s = 0; s < Q; s++) a.lam_f[(int64_t)s * a.g.plane + c] = lam[s];
+   for (int q = 0; q < NP; q++) {
+      const int s = pair_dir(Q, q), o = lat_opp(Q, s);
+      R O;
+      if (q < 3) O = odd[q];
+      else if (q < 9) O = (q - 3) % 2 == 0 ? op[(q - 3) / 2] : om_[(q - 3) / 2];
+      else O = (lat_c(Q, s, 1) > 0 ? op[0] : om_[0]) + (lat_c(Q, s, 2) > 0 ? odd[2] : -odd[2]);
+      const R X = al * p[q] + even, Y = be * d[q] + O;
+      lam[(int64_t)s * plane + c] = X + Y;
+      lam[(int64_t)o * plane + c] = X - Y;
+   }
    if (a.grad_force) {
 #pragma unroll
-      for (int d = 0; d < 3; d++) a.grad_force[(int64_t)d * a.g.plane + c] += (double)gF[d];
+      for (int k = 0; k < 3; k++) a.grad_force[(int64_t)k * plane + c] += widen(gF[k]);
    }
-   if (a.grad_porosity) a.grad_porosity[c] += (double)gsig;
+   if (a.grad_porosity) a.grad_porosity[c] += widen(gsig);
 }
 
 // Loss value of the current state (FP64 partial sums per block).
@@ -321,29 +334,32 @@ __global__ void __launch_bounds__(kReduceThreads) loss_partial_kernel(AdjParams 
         c += (int64_t)gridDim.x * blockDim.x) {
       const uint32_t lk = a.links ? a.links[c] : 0u;
       if (lk & kSolidBit) continue;
-      double rho = 0.0, j[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-      for (int s = 0; s < Q; s++) {
-         const double f = load_pop<ST>(a.state, (int64_t)s * a.g.plane + c, lat_w(Q, s));
-         rho += f;
-         j[0] += f * lat_c(Q, s, 0);
-         j[1] += f * lat_c(Q, s, 1);
-         j[2] += f * lat_c(Q, s, 2);
-      }
-      double F[3] = {a.F[0], a.F[1], a.F[2]};
-      if (a.force_field) {
-         F[0] += a.force_field[c];
-         F[1] += a.force_field[a.g.plane + c];
-         F[2] += a.force_field[2 * a.g.plane + c];
-      }
-      double u[3];
-      for (int d = 0; d < 3; d++) u[d] = (j[d] + 0.5 * F[d]) / rho;
+      double W[3] = {a.loss_weight[c], 0.0, 0.0};
       if (a.loss_kind == LBM_LOSS_VELOCITY) {
-         acc += a.loss_weight[c] * u[0] + a.loss_weight[a.g.plane + c] * u[1] +
-                a.loss_weight[2 * a.g.plane + c] * u[2];
-      } else {
-         acc += a.loss_weight[c] * 0.5 * rho * (u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
+         W[1] = a.loss_weight[a.g.plane + c];
+         W[2] = a.loss_weight[2 * a.g.plane + c];
       }
+      const auto load = [&](int s) { return moment_value<ST>(a.state, (int64_t)s * a.g.plane + c); };
+      const CellMoments<Q, ST, decltype(load)> mom(load);
+      double ff[3] = {0.0, 0.0, 0.0};
+      if (a.force_field) {
+#pragma unroll
+         for (int d = 0; d < 3; d++) ff[d] = a.force_field[d * a.g.plane + c];
+      }
+      // a cell of zero weight adds +-0 as long as its u is finite: a warp of them
+      // (a loss on one plane) leaves out its FP64 operations
+      const bool regular = mom.regular() && finite_bits(ff[0]) && finite_bits(ff[1]) && finite_bits(ff[2]);
+      if (!__any_sync(__activemask(), !regular || W[0] != 0.0 || W[1] != 0.0 || W[2] != 0.0)) continue;
+      double rho, j[3], F[3] = {a.F[0], a.F[1], a.F[2]};
+      mom.get(rho, j);
+      if (a.force_field) {
+#pragma unroll
+         for (int d = 0; d < 3; d++) F[d] += ff[d];
+      }
+#pragma unroll
+      for (int d = 0; d < 3; d++) j[d] += 0.5 * F[d];
+      if (a.loss_kind == LBM_LOSS_VELOCITY) acc += (W[0] * j[0] + W[1] * j[1] + W[2] * j[2]) / rho;
+      else acc += W[0] * 0.5 * (j[0] * j[0] + j[1] * j[1] + j[2] * j[2]) / rho;
    }
    __shared__ double sh[kReduceThreads / 32];
    for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xFFFFFFFFu, acc, off);
@@ -370,18 +386,29 @@ __global__ void sum_partials_kernel(const double* partials, int n, double* out)
    if (threadIdx.x == 0) out[0] = sh[0];
 }
 
+// Blocks along x, one row per block: no divisions for the cell's position.
+template <int Q, int ST, typename R>
+cudaError_t launch_adjoint_r(const AdjParams& a, cudaStream_t st)
+{
+   const int bx = a.g.nx >= 128 ? 128 : (a.g.nx + 31) / 32 * 32;
+   const dim3 grid((unsigned)((a.g.nx + bx - 1) / bx), (unsigned)a.g.ny, (unsigned)a.g.nz);
+   AdjParams b = a;
+   b.k = {a.omega, 1.0 - a.omega, 1.0 - 0.5 * a.omega, a.time_weight, {a.F[0], a.F[1], a.F[2]}};
+   b.kf = {(float)b.k.om, (float)b.k.om1, (float)b.k.om2, (float)b.k.tw, {(float)a.F[0], (float)a.F[1], (float)a.F[2]}};
+   adjoint_step_kernel<Q, ST, R><<<grid, bx, 0, st>>>(b);
+   return cudaGetLastError();
+}
+
 template <int Q, int ST>
 cudaError_t launch_adjoint_t(const AdjParams& a, cudaStream_t st)
 {
-   adjoint_step_kernel<Q, ST><<<(unsigned)((a.g.ncell + 127) / 128), 128, 0, st>>>(a);
-   return cudaGetLastError();
+   return launch_adjoint_r<Q, ST, double>(a, st);
 }
 
 template <int Q, int ST>
 cudaError_t launch_adjoint_f32_t(const AdjParams& a, cudaStream_t st)
 {
-   adjoint_step_f32_kernel<Q, ST><<<(unsigned)((a.g.ncell + 255) / 256), 256, 0, st>>>(a);
-   return cudaGetLastError();
+   return launch_adjoint_r<Q, ST, float>(a, st);
 }
 
 template <int Q, int ST>

@@ -7,6 +7,12 @@
 
 namespace lbm {
 
+// Launch constants of the adjoint in its arithmetic, made on the host.
+template <typename R>
+struct AdjConsts {
+   R om, om1, om2, tw, F[3];   // omega, 1 - omega, 1 - omega/2, time weight, uniform force
+};
+
 struct AdjParams {
    GridDims g;
    double omega;
@@ -14,6 +20,10 @@ struct AdjParams {
    const uint32_t* links;
    const double* force_field;     // planar [3][plane] or null
    const double* porosity;        // [plane] or null
+   // FP32 copies of the fields for the FP32 adjoint, where they hold what it would
+   // round the FP64 ones to (the force field only without a uniform force), or null
+   const float* force_field_f;
+   const float* porosity_f;
    const void* state;             // f^t, the handle's storage, slot s = direction s
    const double* lam_next;        // [Q][plane]
    double* lam;                   // [Q][plane]
@@ -25,6 +35,8 @@ struct AdjParams {
    int collide;                   // 0: loss term only (the last state of a rollout)
    const float* lam_next_f;       // FP32 adjoint: [Q][plane]
    float* lam_f;                  // FP32 adjoint: [Q][plane]
+   AdjConsts<double> k;           // set by the launch functions
+   AdjConsts<float> kf;
 };
 
 cudaError_t launch_adjoint(int Q, int storage, const AdjParams& a, cudaStream_t stream);

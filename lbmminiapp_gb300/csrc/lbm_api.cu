@@ -1014,6 +1014,9 @@ static AdjParams adj_params(const lbm_handle* h, const void* state)
    a.links = h->links;
    a.force_field = h->force_field;
    a.porosity = h->porosity;
+   if (h->force_field && h->cfg.force[0] == 0.0 && h->cfg.force[1] == 0.0 && h->cfg.force[2] == 0.0)
+      a.force_field_f = h->force_field_f;
+   if (h->porosity) a.porosity_f = h->porosity_f;
    a.state = state ? state : readout_buffer(h);
    return a;
 }
