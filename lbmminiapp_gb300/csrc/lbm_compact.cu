@@ -34,6 +34,7 @@ namespace lbm {
 namespace {
 
 constexpr int kCompactWarps = 8;
+constexpr int kCompactBlocks = 2;   // per SM
 
 // Two consecutive stored elements as one word: the even step's copy unit.
 template <typename T> struct PairWord;
@@ -376,13 +377,16 @@ cudaError_t persistent_grid(Kern kern, size_t smem, std::atomic<int>* cache, int
    if (cached == 0) {
       e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
+      e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, carveout_percent(kCompactBlocks, smem));
+      if (e != cudaSuccess) return e;
       int per_sm = 0, nsm = 0;
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kCompactWarps * 32, smem);
       if (e != cudaSuccess) return e;
       e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
       if (e != cudaSuccess) return e;
       if (per_sm < 1) return cudaErrorInvalidConfiguration;
-      cached = per_sm * nsm;
+      // no more than the carve-out is meant for
+      cached = (per_sm < kCompactBlocks ? per_sm : kCompactBlocks) * nsm;
       cache[dev].store(cached, std::memory_order_relaxed);
    }
    grid = cached;
@@ -426,24 +430,50 @@ cudaError_t launch_step_f(int kind, const KParams& p, const CompactGeom& g, void
 }
 
 // ------------------------------------------------------------ copies
+// One direction plane per grid row, four cells per thread at the block's stride:
+// every access is contiguous over a warp (but for the gaps of the solid cells)
+// and the four are in flight together.  One thread per cell looping over the
+// planes moved 1.5 TB/s (143 us for D3Q27 FP16 on 160^3).
+constexpr int kCopyCells = 4;
+
 template <typename T>
-__global__ void expand_kernel(const uint32_t* dcell, uint32_t nf, uint32_t cplane, int Q, const T* cbuf, T* dense,
-                              int64_t plane)
+__global__ void __launch_bounds__(256) expand_kernel(const uint32_t* dcell, uint32_t nf, uint32_t cplane, const T* cbuf,
+                                                     T* dense, int64_t plane)
 {
-   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-   if (i >= nf) return;
-   const int64_t c = dcell[i];
-   for (int s = 0; s < Q; s++) dense[(int64_t)s * plane + c] = cbuf[(uint64_t)s * cplane + i];
+   const uint32_t i0 = blockIdx.x * (256u * kCopyCells) + threadIdx.x;
+   const T* src = cbuf + (uint64_t)blockIdx.y * cplane;
+   T* dst = dense + (int64_t)blockIdx.y * plane;
+   uint32_t c[kCopyCells];
+   T v[kCopyCells];
+#pragma unroll
+   for (int k = 0; k < kCopyCells; k++) {
+      const uint32_t i = i0 + 256u * k;
+      if (i < nf) {
+         c[k] = dcell[i];
+         v[k] = src[i];
+      }
+   }
+#pragma unroll
+   for (int k = 0; k < kCopyCells; k++)
+      if (i0 + 256u * k < nf) dst[c[k]] = v[k];
 }
 
 template <typename T>
-__global__ void compress_kernel(const uint32_t* dcell, uint32_t nf, uint32_t cplane, int Q, const T* dense,
-                                int64_t plane, T* cbuf)
+__global__ void __launch_bounds__(256) compress_kernel(const uint32_t* dcell, uint32_t nf, uint32_t cplane,
+                                                       const T* dense, int64_t plane, T* cbuf)
 {
-   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-   if (i >= nf) return;
-   const int64_t c = dcell[i];
-   for (int s = 0; s < Q; s++) cbuf[(uint64_t)s * cplane + i] = dense[(int64_t)s * plane + c];
+   const uint32_t i0 = blockIdx.x * (256u * kCopyCells) + threadIdx.x;
+   const T* src = dense + (int64_t)blockIdx.y * plane;
+   T* dst = cbuf + (uint64_t)blockIdx.y * cplane;
+   T v[kCopyCells];
+#pragma unroll
+   for (int k = 0; k < kCopyCells; k++) {
+      const uint32_t i = i0 + 256u * k;
+      if (i < nf) v[k] = src[dcell[i]];
+   }
+#pragma unroll
+   for (int k = 0; k < kCopyCells; k++)
+      if (i0 + 256u * k < nf) dst[i0 + 256u * k] = v[k];
 }
 
 __global__ void gather_links_kernel(const OddTile* tiles, uint32_t ntiles, const uint32_t* dcell,
@@ -463,6 +493,11 @@ __global__ void gather_links_kernel(const OddTile* tiles, uint32_t ntiles, const
 }
 
 unsigned blocks_of(uint32_t n) { return (n + 255) / 256; }
+dim3 copy_grid(uint32_t nf, int Q)
+{
+   const uint32_t per = 256u * kCopyCells;
+   return dim3(nf / per + (nf % per ? 1u : 0u), (unsigned)Q);
+}
 
 }  // namespace
 
@@ -492,11 +527,11 @@ cudaError_t launch_compact_expand(int Q, int storage, const uint32_t* dcell, uin
 {
    if (nf == 0) return cudaSuccess;
    if (storage == ST_F32)
-      expand_kernel<uint32_t><<<blocks_of(nf), 256, 0, stream>>>(dcell, nf, cplane, Q, (const uint32_t*)cbuf,
-                                                                  (uint32_t*)dense, plane);
+      expand_kernel<uint32_t><<<copy_grid(nf, Q), 256, 0, stream>>>(dcell, nf, cplane, (const uint32_t*)cbuf,
+                                                                     (uint32_t*)dense, plane);
    else
-      expand_kernel<uint16_t><<<blocks_of(nf), 256, 0, stream>>>(dcell, nf, cplane, Q, (const uint16_t*)cbuf,
-                                                                  (uint16_t*)dense, plane);
+      expand_kernel<uint16_t><<<copy_grid(nf, Q), 256, 0, stream>>>(dcell, nf, cplane, (const uint16_t*)cbuf,
+                                                                     (uint16_t*)dense, plane);
    return cudaGetLastError();
 }
 
@@ -505,11 +540,11 @@ cudaError_t launch_compact_compress(int Q, int storage, const uint32_t* dcell, u
 {
    if (nf == 0) return cudaSuccess;
    if (storage == ST_F32)
-      compress_kernel<uint32_t><<<blocks_of(nf), 256, 0, stream>>>(dcell, nf, cplane, Q, (const uint32_t*)dense,
-                                                                    plane, (uint32_t*)cbuf);
+      compress_kernel<uint32_t><<<copy_grid(nf, Q), 256, 0, stream>>>(dcell, nf, cplane, (const uint32_t*)dense, plane,
+                                                                       (uint32_t*)cbuf);
    else
-      compress_kernel<uint16_t><<<blocks_of(nf), 256, 0, stream>>>(dcell, nf, cplane, Q, (const uint16_t*)dense,
-                                                                    plane, (uint16_t*)cbuf);
+      compress_kernel<uint16_t><<<copy_grid(nf, Q), 256, 0, stream>>>(dcell, nf, cplane, (const uint16_t*)dense, plane,
+                                                                       (uint16_t*)cbuf);
    return cudaGetLastError();
 }
 
