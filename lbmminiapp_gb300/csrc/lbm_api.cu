@@ -17,6 +17,7 @@
 #include "lbm_compact.cuh"
 #include "lbm_dispatch.cuh"
 #include "lbm_f64x.cuh"
+#include "lbm_macros.cuh"
 
 using namespace lbm;
 
@@ -42,7 +43,7 @@ struct lbm_handle {
    cudaEvent_t chunk_ready[2] = {nullptr, nullptr};
    cudaEvent_t chunk_free[2] = {nullptr, nullptr};
    double* partials = nullptr;     // reduction scratch: plane partials or 4 doubles per loss block
-   double* reduce_out = nullptr;   // 4 doubles
+   double* reduce_out = nullptr;   // 4 doubles, host memory that the reductions' last kernel writes to
    uint32_t* sched = nullptr;      // tile counter of the persistent step kernels (zero between launches)
    cudaStream_t stream = nullptr;
    // Compact fluid-only storage (cfg.compact): the steps run on cbuf; buf[0]
@@ -245,8 +246,14 @@ struct Macros {
    static void run(const lbm_handle* h, int64_t c0, int64_t count, const void* buf, int mode, double* rho,
                    double* u, int64_t out_stride)
    {
-      macros_kernel<Q, ST><<<blocks_for(count, 256), 256, 0, h->stream>>>(dims_of(h), c0, count, buf, h->links,
-                                                                           mode, rho, u, out_stride);
+      const unsigned blocks = blocks_for(count, 256);
+      const GridDims g = dims_of(h);
+      if (mode == 0)
+         macros_kernel<Q, ST, 0><<<blocks, 256, 0, h->stream>>>(g, c0, count, buf, h->links, rho, u, out_stride);
+      else if (mode == 1)
+         macros_kernel<Q, ST, 1><<<blocks, 256, 0, h->stream>>>(g, c0, count, buf, h->links, rho, u, out_stride);
+      else
+         macros_kernel<Q, ST, 2><<<blocks, 256, 0, h->stream>>>(g, c0, count, buf, h->links, rho, u, out_stride);
    }
 };
 
@@ -255,10 +262,14 @@ struct Conserved {
    static void run(const lbm_handle* h, const void* buf, int mode, double* partials, double* out)
    {
       PlanePartial* part = reinterpret_cast<PlanePartial*>(partials);
-      const int64_t per_range = plane_per_range(h->ncell);
+      const int64_t per_range = plane_per_range(Q, h->ncell);
       const int nblocks = plane_blocks(Q, h->ncell);
-      conserved_plane_kernel<Q, ST><<<nblocks, kReduceThreads, 0, h->stream>>>(dims_of(h), buf, h->links, mode,
-                                                                              per_range, part);
+      if (h->links)
+         conserved_plane_kernel<Q, ST, true><<<nblocks, kReduceThreads, 0, h->stream>>>(dims_of(h), buf, h->links,
+                                                                                       mode, per_range, part);
+      else
+         conserved_plane_kernel<Q, ST, false><<<nblocks, kReduceThreads, 0, h->stream>>>(dims_of(h), buf, nullptr,
+                                                                                        mode, per_range, part);
       conserved_plane_final_kernel<Q><<<1, kReduceThreads, 0, h->stream>>>(part, nblocks, mode, out);
    }
 };
@@ -440,7 +451,7 @@ void lbm_destroy(lbm_handle* h)
       if (h->chunk_free[k]) cudaEventDestroy(h->chunk_free[k]);
    }
    cudaFree(h->partials);
-   cudaFree(h->reduce_out);
+   cudaFreeHost(h->reduce_out);
    cudaFree(h->sched);
    cudaFree(h->cbuf);
    cudaFree(h->dcell);
@@ -519,7 +530,15 @@ lbm_status lbm_create(const lbm_config* cfg, lbm_handle** out)
       const size_t loss_bytes = sizeof(double) * 4 * kReduceBlocks;
       st = dev_alloc(h, (void**)&h->partials, plane_bytes > loss_bytes ? plane_bytes : loss_bytes);
    }
-   if (st == LBM_OK) st = dev_alloc(h, (void**)&h->reduce_out, sizeof(double) * 4);
+   if (st == LBM_OK) {
+      // written by kernels over the host link: no copy after a reduction
+      const cudaError_t e = cudaHostAlloc((void**)&h->reduce_out, sizeof(double) * 4, cudaHostAllocPortable);
+      if (e != cudaSuccess) {
+         cudaGetLastError();
+         h->reduce_out = nullptr;
+         st = fail(h, LBM_ERR_OUT_OF_MEMORY, "cudaHostAlloc: %s", cudaGetErrorString(e));
+      }
+   }
    if (st == LBM_OK) st = dev_alloc(h, (void**)&h->sched, 4 * kFeedWords);
    if (st == LBM_OK) {
       const cudaError_t e = cudaMemset(h->sched, 0, 4 * kFeedWords);
@@ -843,6 +862,20 @@ lbm_status lbm_step(lbm_handle* h, int nsteps)
    return LBM_OK;
 }
 
+// Device address of `n` doubles of page-locked host memory, null for any other
+// memory.
+static double* mapped_host(double* p, int64_t n)
+{
+   cudaPointerAttributes a, b;
+   if (cudaPointerGetAttributes(&a, p) != cudaSuccess || cudaPointerGetAttributes(&b, p + (n - 1)) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+   }
+   if (a.type != cudaMemoryTypeHost || b.type != cudaMemoryTypeHost || !a.devicePointer || !b.devicePointer) return nullptr;
+   double* d = static_cast<double*>(a.devicePointer);
+   return static_cast<double*>(b.devicePointer) == d + (n - 1) ? d : nullptr;
+}
+
 lbm_status lbm_get_macros(lbm_handle* h, double* rho, double* u)
 {
    if (!h || !rho || !u) return LBM_ERR_INVALID_ARGUMENT;
@@ -851,9 +884,19 @@ lbm_status lbm_get_macros(lbm_handle* h, double* rho, double* u)
    // from the stored buffer (src/propagation/PropagationAB.cpp:222-281).
    const int mode = h->cfg.prop_pattern == LBM_PATTERN_AA ? logical_mode(h) : 0;
    lbm_status st = dense_for_read(h);
-   if (st == LBM_OK) st = ensure_copy_stream(h);
    if (st != LBM_OK) return st;
    const int64_t n = h->ncell;
+   // Page-locked arrays are written by the kernel itself over the host link.
+   double* mrho = mapped_host(rho, n);
+   double* mu = mrho ? mapped_host(u, 3 * n) : nullptr;
+   if (mu) {
+      dispatch_q_st<Macros>(h->Q, h->storage, h, (int64_t)0, n, readout_buffer(h), mode, mrho, mu, n);
+      LBM_CUDA(h, cudaGetLastError());
+      LBM_CUDA(h, cudaStreamSynchronize(h->stream));
+      return LBM_OK;
+   }
+   st = ensure_copy_stream(h);
+   if (st != LBM_OK) return st;
    const int64_t chunk = chunk_cells(h, 4);
    const size_t half = h->staging_elems / 2;
    const void* buf = readout_buffer(h);
@@ -887,8 +930,8 @@ lbm_status lbm_reduce_conserved(lbm_handle* h, double out[4])
    dispatch_q_st<Conserved>(h->Q, h->storage, h, readout_buffer(h), logical_mode(h), h->partials,
                             h->reduce_out);
    LBM_CUDA(h, cudaGetLastError());
-   LBM_CUDA(h, cudaMemcpyAsync(out, h->reduce_out, sizeof(double) * 4, cudaMemcpyDeviceToHost, h->stream));
    LBM_CUDA(h, cudaStreamSynchronize(h->stream));
+   std::memcpy(out, h->reduce_out, sizeof(double) * 4);
    for (int k = 0; k < 4; k++)
       if (!std::isfinite(out[k])) return fail(h, LBM_ERR_DIVERGED, "conserved sum %d is %g", k, out[k]);
    return LBM_OK;
@@ -1036,8 +1079,8 @@ lbm_status lbm_loss(lbm_handle* h, const void* state, int loss_kind, const doubl
    a.loss_weight = weight;
    a.time_weight = time_weight;
    LBM_CUDA(h, launch_loss(h->Q, h->storage, a, h->partials, kReduceBlocks, h->reduce_out, h->stream));
-   LBM_CUDA(h, cudaMemcpyAsync(out_host, h->reduce_out, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
    LBM_CUDA(h, cudaStreamSynchronize(h->stream));
+   *out_host = h->reduce_out[0];
    return LBM_OK;
 }
 

@@ -226,58 +226,6 @@ __global__ void export_plane_kernel(GridDims g, const void* buf, const uint32_t*
    dst[c] = load_pop<ST>(buf, idx, w);
 }
 
-// Logical population of direction s at cell c (same modes as export).
-template <int Q, int ST>
-__device__ __forceinline__ double logical_pop(const GridDims& g, const void* buf, uint32_t lk, int x, int y,
-                                              int z, int64_t c, int s, int mode)
-{
-   const int o = lat_opp(Q, s);
-   if (mode == 0) return load_pop<ST>(buf, (int64_t)s * g.plane + c, lat_w(Q, s));
-   if (mode == 1 || s == lat_rest(Q) || ((lk >> o) & 1u))
-      return load_pop<ST>(buf, (int64_t)o * g.plane + c, lat_w(Q, o));
-   const int64_t n = nbr_cell(g, x, y, z, -lat_c(Q, s, 0), -lat_c(Q, s, 1), -lat_c(Q, s, 2));
-   return load_pop<ST>(buf, (int64_t)s * g.plane + n, lat_w(Q, s));
-}
-
-// rho and u = sum(c f)/rho (no F/2 shift) for the cells [c0, c0+count);
-// cell c0+k goes to rho[k] and u[d*out_stride + k]; NaN at solid cells.
-// Zero stencil terms are left out and +-1 terms become adds or subtracts,
-// which gives the same sums as the reference's f * c accumulation.
-template <int Q, int ST>
-__global__ void macros_kernel(GridDims g, int64_t c0, int64_t count, const void* buf, const uint32_t* links,
-                              int mode, double* rho, double* u, int64_t out_stride)
-{
-   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-   if (k >= count) return;
-   const int64_t c = c0 + k;
-   int x, y, z;
-   if (!cell_xyz(g, c, x, y, z)) return;
-   const uint32_t lk = links ? links[c] : 0u;
-   if (lk & kSolidBit) {
-      const double nan = __longlong_as_double(0x7FF8000000000000LL);
-      rho[k] = nan;
-      u[k] = u[out_stride + k] = u[2 * out_stride + k] = nan;
-      return;
-   }
-   double r = 0.0, m[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-   for (int s = 0; s < Q; s++) {
-      const double f = logical_pop<Q, ST>(g, buf, lk, x, y, z, c, s, mode);
-      r += f;
-#pragma unroll
-      for (int d = 0; d < 3; d++) {
-         const int cd = lat_c(Q, s, d);
-         if (cd > 0) m[d] += f;
-         else if (cd < 0) m[d] -= f;
-      }
-   }
-   const double ir = 1.0 / r;
-   rho[k] = r;
-   u[k] = m[0] * ir;
-   u[out_stride + k] = m[1] * ir;
-   u[2 * out_stride + k] = m[2] * ir;
-}
-
 // FP64 mass / momentum sums over fluid cells, exact for physical states.
 //
 // A population f in [2^-32, 1) -- every population of a physical state -- is
@@ -461,19 +409,24 @@ struct PlanePartial {
    __int128 m, s;   // exact sums, units of 2^-84
    double md, sd;   // FP64 sums of the elements outside [2^-32, 1)
 };
-constexpr int kPlaneRanges = 96;
-constexpr int kPlaneUnroll = 4;
+constexpr int kPlaneRanges = 32;   // D3Q19; one wave of four blocks on each of the 152 SMs
+// Loads in flight bound the kernel: with 4 per thread, and 4 more for the link
+// words it did not have, 128^3 D3Q19 FP64 ran at 3.8 TB/s (84 us).
+constexpr int kPlaneUnroll = 8;
 
-template <int Q, int ST>
-__global__ void __launch_bounds__(kReduceThreads) conserved_plane_kernel(GridDims g, const void* buf,
-                                                                        const uint32_t* links, int mode,
-                                                                        int64_t per_range, PlanePartial* partials)
+// x == +-0, without the FP64 pipe.
+__device__ __forceinline__ bool zero_bits(double x) { return (__double_as_longlong(x) << 1) == 0; }
+
+template <int Q, int ST, bool LINKS>
+__global__ void __launch_bounds__(kReduceThreads, 4) conserved_plane_kernel(GridDims g, const void* buf,
+                                                                           const uint32_t* links, int mode,
+                                                                           int64_t per_range, PlanePartial* partials)
 {
    const int r = (int)(blockIdx.x % Q);
    const int64_t c0 = (int64_t)(blockIdx.x / Q) * per_range;
    const int64_t c1 = c0 + per_range < g.ncell ? c0 + per_range : g.ncell;
-   const double w = weight_at<Q>(r);
-   const bool signed_links = mode == 2 && links != nullptr;
+   const double w = ST == ST_F64 ? 0.0 : weight_at<Q>(r);
+   const bool signed_links = LINKS && mode == 2;
    Acc128 am, an;   // all elements; those with link bit r set (mode 2 only)
    acc_zero(am);
    acc_zero(an);
@@ -483,7 +436,7 @@ __global__ void __launch_bounds__(kReduceThreads) conserved_plane_kernel(GridDim
 #pragma unroll
       for (int u = 0; u < kPlaneUnroll; u++) {
          const int64_t c = cb + (int64_t)u * blockDim.x;
-         lk[u] = c < c1 ? (links ? links[c] : 0u) : kSolidBit;
+         lk[u] = c < c1 ? (LINKS ? links[c] : 0u) : kSolidBit;
       }
       double f[kPlaneUnroll];
 #pragma unroll
@@ -521,13 +474,19 @@ __global__ void __launch_bounds__(kReduceThreads) conserved_plane_kernel(GridDim
    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
    // signed sums: all minus twice the flipped ones
    __int128 m = acc_value(am), sg = m - 2 * acc_value(an);
-   double sd = md - 2.0 * nd;
 #pragma unroll
    for (int off = 16; off > 0; off >>= 1) {
       m += shfl_down_i128(m, off);
       sg += shfl_down_i128(sg, off);
-      md += __shfl_down_sync(0xFFFFFFFFu, md, off);
-      sd += __shfl_down_sync(0xFFFFFFFFu, sd, off);
+   }
+   double sd = 0.0;
+   if (__any_sync(0xFFFFFFFFu, !(zero_bits(md) && zero_bits(nd)))) {
+      sd = md - 2.0 * nd;
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) {
+         md += __shfl_down_sync(0xFFFFFFFFu, md, off);
+         sd += __shfl_down_sync(0xFFFFFFFFu, sd, off);
+      }
    }
    if (lane == 0) {
       shx[0][warp] = m;
@@ -541,24 +500,29 @@ __global__ void __launch_bounds__(kReduceThreads) conserved_plane_kernel(GridDim
       for (int k = 0; k < kReduceThreads / 32; k++) {
          pp.m += shx[0][k];
          pp.s += shx[1][k];
-         pp.md += shd[0][k];
-         pp.sd += shd[1][k];
+         if (!(zero_bits(shd[0][k]) && zero_bits(shd[1][k]))) {
+            pp.md += shd[0][k];
+            pp.sd += shd[1][k];
+         }
       }
       partials[blockIdx.x] = pp;
    }
 }
 
 // Cells per range of conserved_plane_kernel (a multiple of the unrolled
-// block stride) and the number of blocks it launches.
-inline int64_t plane_per_range(int64_t ncell)
+// block stride) and the number of blocks it launches: one wave, so no last one
+// that is nearly empty, and a third of the partials for the last kernel.
+inline int64_t plane_per_range(int Q, int64_t ncell)
 {
    const int64_t step = (int64_t)kPlaneUnroll * kReduceThreads;
-   int64_t per = (ncell + kPlaneRanges - 1) / kPlaneRanges;
+   const int ranges = kPlaneRanges * 19 / Q;
+   const int64_t per = (ncell + ranges - 1) / ranges;
    return (per + step - 1) / step * step;
 }
 inline int plane_blocks(int Q, int64_t ncell)
 {
-   return Q * (int)((ncell + plane_per_range(ncell) - 1) / plane_per_range(ncell));
+   const int64_t per = plane_per_range(Q, ncell);
+   return Q * (int)((ncell + per - 1) / per);
 }
 
 // Nearest double to v (to within one rounding of the low word).
@@ -598,19 +562,24 @@ static __global__ void conserved_final_kernel(const ConservedPartial* partials, 
 }
 
 // Totals from the plane partials of conserved_plane_kernel (nblocks of
-// them, plane b mod Q): out = {mass, momentum x, y, z}.
+// them, plane b mod Q): out = {mass, momentum x, y, z}.  The FP64 sums are
+// made only when a partial has one (12 us of FP64 pipe otherwise).
 template <int Q>
-__global__ void conserved_plane_final_kernel(const PlanePartial* partials, int nblocks, int mode, double* out)
+__global__ void __launch_bounds__(kReduceThreads) conserved_plane_final_kernel(const PlanePartial* partials,
+                                                                              int nblocks, int mode, double* out)
 {
    __shared__ __int128 shx[4][kReduceThreads];
    __shared__ double shd[4][kReduceThreads];
    __int128 x[4] = {0, 0, 0, 0};
    double d[4] = {0.0, 0.0, 0.0, 0.0};
+   bool any = false;
    for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
       const int r = b % Q;
       const PlanePartial pp = partials[b];
+      const bool inexact = !(zero_bits(pp.md) && zero_bits(pp.sd));
+      any = any || inexact;
       x[0] += pp.m;
-      d[0] += pp.md;
+      if (inexact) d[0] += pp.md;
       // mode 2 uses the signed sums; mode 1 flips every direction
       const __int128 xm = mode == 2 ? pp.s : pp.m;
       const double dm = mode == 2 ? pp.sd : pp.md;
@@ -619,13 +588,14 @@ __global__ void conserved_plane_final_kernel(const PlanePartial* partials, int n
          const int cr = (mode == 1 ? -1 : 1) * velocity_at<Q>(r, e);
          if (cr > 0) {
             x[1 + e] += xm;
-            d[1 + e] += dm;
+            if (inexact) d[1 + e] += dm;
          } else if (cr < 0) {
             x[1 + e] -= xm;
-            d[1 + e] -= dm;
+            if (inexact) d[1 + e] -= dm;
          }
       }
    }
+   const bool fp64 = __syncthreads_or(any);
 #pragma unroll
    for (int k = 0; k < 4; k++) {
       shx[k][threadIdx.x] = x[k];
@@ -636,7 +606,7 @@ __global__ void conserved_plane_final_kernel(const PlanePartial* partials, int n
       if ((int)threadIdx.x < stride)
          for (int k = 0; k < 4; k++) {
             shx[k][threadIdx.x] += shx[k][threadIdx.x + stride];
-            shd[k][threadIdx.x] += shd[k][threadIdx.x + stride];
+            if (fp64) shd[k][threadIdx.x] += shd[k][threadIdx.x + stride];
          }
       __syncthreads();
    }
