@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(kSparseThreads, sparse_min_blocks<Q>()) sparse
    };
    if constexpr (AR == AR_F64) {
       auto in = [&](int s) { return d[s]; };
-      collide_f64_uniform<Q>(in, put, 0.0, p);
+      collide_f64_uniform<Q, true>(in, put, 0.0, p);
    } else {
       uint64_t bits[Q];
 #pragma unroll

@@ -19,7 +19,7 @@
 //            from src, write own slot s in tgt
 #pragma once
 
-#include "lbm_f64x.cuh"
+#include "lbm_f64x_cell.cuh"
 #include "lbm_launch.cuh"
 #include "lbm_physics.cuh"
 
@@ -136,9 +136,10 @@ __device__ __forceinline__ void cell_force_f32(const KParams& p, int64_t c, floa
    }
 }
 
-// One launch = one time step (or one range of it) of one propagation kind.
+// One launch = one time step (or one range of it) of one propagation kind.  The
+// exact FP64 arithmetic needs 16 warps per SM to keep its two pipes busy.
 template <int Q, int ST, int AR, int KIND, bool LINKS, bool FIELDS, typename IT>
-__global__ void __launch_bounds__(256) step_kernel(const KParams p, const typename Store<ST>::T* src,
+__global__ void __launch_bounds__(256, AR == AR_F64 ? 2 : 1) step_kernel(const KParams p, const typename Store<ST>::T* src,
                                                    typename Store<ST>::T* dst)
 {
    wait_prior_grid();
@@ -161,8 +162,8 @@ __global__ void __launch_bounds__(256) step_kernel(const KParams p, const typena
       cell_force_f64<FIELDS>(p, ci.c, F0, F1, F2, sp);
       auto in = [&](int s) { return d[s]; };
       auto out = [&](int s, double v) { *slot_ptr(dbase, pb, write_access<Q, KIND, LINKS>(ci, lk, s)) = v; };
-      if (FIELDS && p.force_field) collide_f64_emit<Q, XF_CELL>(in, out, F0, F1, F2, sp, p);
-      else collide_f64_uniform<Q>(in, out, sp, p);
+      if constexpr (FIELDS) collide_f64_emit<Q, XF_CELL, true>(in, out, F0, F1, F2, sp, p);
+      else collide_f64_uniform<Q, true>(in, out, sp, p);
    } else if constexpr (AR == AR_F64X) {
       uint64_t bits[Q];
       const unsigned long long* s64 = reinterpret_cast<const unsigned long long*>(sbase);
