@@ -43,7 +43,10 @@ struct lbm_handle {
    cudaEvent_t chunk_ready[2] = {nullptr, nullptr};
    cudaEvent_t chunk_free[2] = {nullptr, nullptr};
    double* partials = nullptr;     // reduction scratch: plane partials or 4 doubles per loss block
-   double* reduce_out = nullptr;   // 4 doubles, host memory that the reductions' last kernel writes to
+   double* reduce_out = nullptr;   // 4 doubles
+   // The grid and the collision constants, which no call changes: made once, not at
+   // each launch (a step of a small box is bound by its launch).
+   KParams params = {};
    uint32_t* sched = nullptr;      // tile counter of the persistent step kernels (zero between launches)
    cudaStream_t stream = nullptr;
    // Compact fluid-only storage (cfg.compact): the steps run on cbuf; buf[0]
@@ -136,8 +139,7 @@ void dev_free(lbm_handle* h, void* p, size_t bytes)
 // Step-kernel parameters for the cell range [start, end).
 KParams make_params(const lbm_handle* h, int64_t start, int64_t end, Launch& L)
 {
-   KParams p;
-   std::memset(&p, 0, sizeof(p));
+   KParams p = h->params;
    const lbm_config& c = h->cfg;
    p.nx = c.nx;
    p.ny = c.ny;
@@ -149,8 +151,6 @@ KParams make_params(const lbm_handle* h, int64_t start, int64_t end, Launch& L)
    const int64_t nxy = (int64_t)c.nx * c.ny;
    const int64_t z0 = start / nxy, z1 = (end - 1) / nxy + 1;
    p.z0 = (int)z0;
-   set_collision_constants(p, h->Q, c.omega, c.force,
-                           (c.unroll && h->Q == 19 && c.prop_pattern == LBM_PATTERN_AA) ? 1 : 0);
    p.links = h->links;
    p.force_field = h->force_field;
    p.force_field_f = h->force_field_f;
@@ -451,7 +451,7 @@ void lbm_destroy(lbm_handle* h)
       if (h->chunk_free[k]) cudaEventDestroy(h->chunk_free[k]);
    }
    cudaFree(h->partials);
-   cudaFreeHost(h->reduce_out);
+   cudaFree(h->reduce_out);
    cudaFree(h->sched);
    cudaFree(h->cbuf);
    cudaFree(h->dcell);
@@ -511,6 +511,8 @@ lbm_status lbm_create(const lbm_config* cfg, lbm_handle** out)
       const int64_t align = 512 / h->elem;
       h->plane = (ncell + align - 1) / align * align;
       h->buffer_bytes = (uint64_t)h->plane * h->Q * h->elem;
+      set_collision_constants(h->params, h->Q, c.omega, c.force,
+                              (c.unroll && h->Q == 19 && c.prop_pattern == LBM_PATTERN_AA) ? 1 : 0);
    }
    if (st == LBM_OK) {
       int ndev = 0;
@@ -530,15 +532,7 @@ lbm_status lbm_create(const lbm_config* cfg, lbm_handle** out)
       const size_t loss_bytes = sizeof(double) * 4 * kReduceBlocks;
       st = dev_alloc(h, (void**)&h->partials, plane_bytes > loss_bytes ? plane_bytes : loss_bytes);
    }
-   if (st == LBM_OK) {
-      // written by kernels over the host link: no copy after a reduction
-      const cudaError_t e = cudaHostAlloc((void**)&h->reduce_out, sizeof(double) * 4, cudaHostAllocPortable);
-      if (e != cudaSuccess) {
-         cudaGetLastError();
-         h->reduce_out = nullptr;
-         st = fail(h, LBM_ERR_OUT_OF_MEMORY, "cudaHostAlloc: %s", cudaGetErrorString(e));
-      }
-   }
+   if (st == LBM_OK) st = dev_alloc(h, (void**)&h->reduce_out, sizeof(double) * 4);
    if (st == LBM_OK) st = dev_alloc(h, (void**)&h->sched, 4 * kFeedWords);
    if (st == LBM_OK) {
       const cudaError_t e = cudaMemset(h->sched, 0, 4 * kFeedWords);
@@ -930,8 +924,8 @@ lbm_status lbm_reduce_conserved(lbm_handle* h, double out[4])
    dispatch_q_st<Conserved>(h->Q, h->storage, h, readout_buffer(h), logical_mode(h), h->partials,
                             h->reduce_out);
    LBM_CUDA(h, cudaGetLastError());
+   LBM_CUDA(h, cudaMemcpyAsync(out, h->reduce_out, sizeof(double) * 4, cudaMemcpyDeviceToHost, h->stream));
    LBM_CUDA(h, cudaStreamSynchronize(h->stream));
-   std::memcpy(out, h->reduce_out, sizeof(double) * 4);
    for (int k = 0; k < 4; k++)
       if (!std::isfinite(out[k])) return fail(h, LBM_ERR_DIVERGED, "conserved sum %d is %g", k, out[k]);
    return LBM_OK;
@@ -1079,8 +1073,8 @@ lbm_status lbm_loss(lbm_handle* h, const void* state, int loss_kind, const doubl
    a.loss_weight = weight;
    a.time_weight = time_weight;
    LBM_CUDA(h, launch_loss(h->Q, h->storage, a, h->partials, kReduceBlocks, h->reduce_out, h->stream));
+   LBM_CUDA(h, cudaMemcpyAsync(out_host, h->reduce_out, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
    LBM_CUDA(h, cudaStreamSynchronize(h->stream));
-   *out_host = h->reduce_out[0];
    return LBM_OK;
 }
 

@@ -123,6 +123,44 @@ __device__ __forceinline__ void pairs_exact(const ExactCell& c, const In& in, Em
    }
 }
 
+// rho and sum c f, added up direction by direction as the reference does and
+// rounded after every addition, in integer instructions; in(s) gives the pattern
+// of population s.  False (the results mean nothing) unless the populations lie in
+// [2^-10, 1/4), the rest one below 1, and rho < 2.
+template <int Q, class In>
+__device__ __forceinline__ bool sums_soft(const In& in, double& rho, double (&v)[3])
+{
+   constexpr uint32_t kLeast = (uint32_t)(1023 - 10) << 20, kQuarter = (uint32_t)(1023 - 2) << 20,
+                      kOne = (uint32_t)1023 << 20;
+   uint32_t least = kQuarter, most = 0u, wrapped = 0u;
+   uint64_t r = 0;
+   int64_t j[3] = {0, 0, 0};
+#pragma unroll
+   for (int s = 0; s < Q; s++) {
+      const uint64_t b = in(s);
+      const uint32_t hi = (uint32_t)(b >> 32);
+      least = least < hi ? least : hi;
+      if (s != lat_rest(Q)) most = most > hi ? most : hi;
+      else wrapped |= hi >= kOne ? 0x80000000u : 0u;
+      const uint64_t X = soft::image(b);
+      r = s == 0 ? X : soft::round_positive(r + X);
+      // rho < 2: looked at often enough that the sum cannot wrap in between
+      if (s % 6 == 5 || s == Q - 1) wrapped |= (uint32_t)(r >> 32);
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+         const int cs = lat_c(Q, s, k);
+         const bool first = s == 2 * k;   // the axis pairs come first, +e_k at 2k
+         if (cs > 0) j[k] = first ? (int64_t)X : soft::round_signed((int64_t)((uint64_t)j[k] + X));
+         else if (cs < 0) j[k] = soft::round_signed((int64_t)((uint64_t)j[k] - X));
+      }
+   }
+   if (least < kLeast || most >= kQuarter || (wrapped & 0x80000000u)) return false;
+   rho = soft::positive_to_double(r);
+#pragma unroll
+   for (int k = 0; k < 3; k++) v[k] = soft::signed_to_double(j[k]);
+   return true;
+}
+
 // One cell: in(s) gives population s (called twice per direction), emit(s, out)
 // takes the results.  F is read for XF_CELL only.  SOFT: returns false, with
 // nothing emitted, for a cell outside the integer additions' ranges.
@@ -135,35 +173,7 @@ __device__ __forceinline__ bool collide_f64_form(const In& in, Emit& emit, doubl
    double rho = 0.0;
    c.v[0] = c.v[1] = c.v[2] = 0.0;
    if constexpr (SOFT) {
-      // populations in [2^-10, 1/4), the rest one below 1; rho < 2, looked at often
-      // enough that the sum cannot wrap in between
-      constexpr uint32_t kLeast = (uint32_t)(1023 - 10) << 20, kQuarter = (uint32_t)(1023 - 2) << 20,
-                         kOne = (uint32_t)1023 << 20;
-      uint32_t least = kQuarter, most = 0u, wrapped = 0u;
-      uint64_t r = 0;
-      int64_t j[3] = {0, 0, 0};
-#pragma unroll
-      for (int s = 0; s < Q; s++) {
-         const uint64_t b = x64::double_bits(in(s));
-         const uint32_t hi = (uint32_t)(b >> 32);
-         least = least < hi ? least : hi;
-         if (s != lat_rest(Q)) most = most > hi ? most : hi;
-         else wrapped |= hi >= kOne ? 0x80000000u : 0u;
-         const uint64_t X = soft::image(b);
-         r = s == 0 ? X : soft::round_positive(r + X);
-         if (s % 6 == 5 || s == Q - 1) wrapped |= (uint32_t)(r >> 32);
-#pragma unroll
-         for (int k = 0; k < 3; k++) {
-            const int cs = lat_c(Q, s, k);
-            const bool first = s == 2 * k;   // the axis pairs come first, +e_k at 2k
-            if (cs > 0) j[k] = first ? (int64_t)X : soft::round_signed((int64_t)((uint64_t)j[k] + X));
-            else if (cs < 0) j[k] = soft::round_signed((int64_t)((uint64_t)j[k] - X));
-         }
-      }
-      if (least < kLeast || most >= kQuarter || (wrapped & 0x80000000u)) return false;
-      rho = soft::positive_to_double(r);
-#pragma unroll
-      for (int k = 0; k < 3; k++) c.v[k] = soft::signed_to_double(j[k]);
+      if (!sums_soft<Q>([&](int s) { return x64::double_bits(in(s)); }, rho, c.v)) return false;
    } else {
 #pragma unroll
       for (int s = 0; s < Q; s++) {

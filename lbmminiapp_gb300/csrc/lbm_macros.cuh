@@ -9,12 +9,13 @@ namespace lbm {
 
 // rho and u = sum(c f)/rho (no F/2 shift) for the cells [c0, c0+count);
 // cell c0+k goes to rho[k] and u[d*out_stride + k]; NaN at solid cells.  mode as
-// for export_plane_kernel.  In mode 1 slot s holds direction opp(s): the sums run
-// over the slots and the momentum changes sign.
+// for export_plane_kernel: 0 slot s holds direction s, 1 slot opp(s) does, 2 pull
+// gather.  FP64 storage: the sums are the reference's, rounded after every
+// addition, so that the readout of equal populations is equal text; the shifted
+// formats are summed error-free (CellMoments).
 //
-// Bound by memory and the rest of its FP64 instructions (a reciprocal and three
-// products): the sums are CellMoments'.  At 128^3, D3Q19 FP64: 290 us in chunks
-// when the 49 adds per cell ran on the FP64 pipe.
+// Bound by the host link for page-locked arrays (67 MB at 189 GB/s for 128^3).
+// With the 49 adds per cell on the FP64 pipe the kernel alone took 290 us there.
 template <int Q, int ST, int MODE>
 __global__ void __launch_bounds__(256) macros_kernel(GridDims g, int64_t c0, int64_t count, const void* buf,
                                                      const uint32_t* links, double* rho, double* u, int64_t out_stride)
@@ -42,17 +43,34 @@ __global__ void __launch_bounds__(256) macros_kernel(GridDims g, int64_t c0, int
       ci.dzm = (z == 0) ? (g.nz - 1) * nxy : -nxy;
       ci.dzp = (z == g.nz - 1) ? -(g.nz - 1) * nxy : nxy;
    }
+   // stored value of direction s
    const auto load = [&](int s) {
-      Access a{s, 0};
+      Access a{MODE == 1 ? lat_opp(Q, s) : s, 0};
       if constexpr (MODE == 2) a = read_access<Q, K_AB_PULL, true>(ci, lk, s);
       return moment_value<ST>(buf, (int64_t)a.slot * g.plane + (c + a.off));
    };
-   const CellMoments<Q, ST, decltype(load)> mom(load);
    double r, m[3];
-   mom.get(r, m);
-   double ir = 1.0 / r;
+   if constexpr (ST == ST_F64) {
+      if (!sums_soft<Q>(load, r, m)) {
+         r = m[0] = m[1] = m[2] = 0.0;
+#pragma unroll
+         for (int s = 0; s < Q; s++) {
+            const double f = x64::as_double(load(s));
+            r = __dadd_rn(r, f);
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+               const int cd = lat_c(Q, s, d);
+               if (cd > 0) m[d] = __dadd_rn(m[d], f);
+               else if (cd < 0) m[d] = __dsub_rn(m[d], f);
+            }
+         }
+      }
+   } else {
+      const CellMoments<Q, ST, decltype(load)> mom(load);
+      mom.get(r, m);
+   }
+   const double ir = 1.0 / r;
    rho[k] = r;
-   if constexpr (MODE == 1) ir = -ir;
    u[k] = m[0] * ir;
    u[out_stride + k] = m[1] * ir;
    u[2 * out_stride + k] = m[2] * ir;
