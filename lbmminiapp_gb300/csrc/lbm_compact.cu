@@ -167,13 +167,11 @@ __global__ void __launch_bounds__(kCompactWarps * 32, 2) compact_even_kernel(con
          const uint32_t i0 = t * 64 + 2 * (uint32_t)lane;
          if (i0 < g.nf) {
             const W* sm = mine + stage * Q * 32;
-            float G0[Q], G1[Q];
+            x64::f2 G[Q];
 #pragma unroll
-            for (int s = 0; s < Q; s++) PW::unpack(sm[s * 32 + lane], G0[s], G1[s]);
-            auto emit = [&](int s, float a, float b) {
-               *reinterpret_cast<W*>(buf + (g.soff[s] + i0)) = PW::pack(a, b);
-            };
-            collide2_f32_emit<Q, ST, FORCE>(G0, G1, p, emit);
+            for (int s = 0; s < Q; s++) PW::unpack(sm[s * 32 + lane], G[s].x, G[s].y);
+            auto emit = [&](int s, x64::f2 o) { *reinterpret_cast<W*>(buf + (g.soff[s] + i0)) = PW::pack(o.x, o.y); };
+            collide2_f32_emit<Q, ST, FORCE>(G, p, emit);
          }
          if (t1 >= ntiles) break;
          t = t1;

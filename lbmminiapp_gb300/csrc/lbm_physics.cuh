@@ -16,6 +16,7 @@
 #include <cstdint>
 
 #include "lbm_lattice.cuh"
+#include "lbm_packed.cuh"
 
 namespace lbm {
 
@@ -110,6 +111,9 @@ __host__ __device__ constexpr int pair_rep()
 // S enters only through per-cell factors.  Opposite directions share
 // cu(opp) = -cu, so S (eq - w) = A +- B with A = w (S drho + S rho (cu^2 - uu)/2)
 // and B = w S rho cu.
+// Every operation is written with its own rounding (products joined to sums by
+// explicit multiply-adds), so that the one-cell and the two-cell forms, in any
+// kernel, give the same bits.
 template <int ST> struct ShiftScale { static constexpr float S = 1.0f; };
 template <> struct ShiftScale<ST_F16> { static constexpr float S = kF16Scale; };
 
@@ -160,11 +164,11 @@ __device__ __forceinline__ ShiftedCell shifted_cell(const float (&G)[Q], float F
    c.u3[0] = fmaf(j0, iS, 0.5f * F0) * ir3;
    c.u3[1] = fmaf(j1, iS, 0.5f * F1) * ir3;
    c.u3[2] = fmaf(j2, iS, 0.5f * F2) * ir3;
-   c.uu = (c.u3[0] * c.u3[0] + c.u3[1] * c.u3[1] + c.u3[2] * c.u3[2]) * (1.0f / 3.0f);   // 3 u.u
+   c.uu = fmaf(c.u3[2], c.u3[2], fmaf(c.u3[0], c.u3[0], x64::fmul(c.u3[1], c.u3[1]))) * (1.0f / 3.0f);   // 3 u.u
    c.F3[0] = 3.0f * F0;
    c.F3[1] = 3.0f * F1;
    c.F3[2] = 3.0f * F2;
-   c.fu = FORCE ? (c.F3[0] * c.u3[0] + c.F3[1] * c.u3[1] + c.F3[2] * c.u3[2]) * (1.0f / 3.0f) : 0.0f;
+   c.fu = FORCE ? fmaf(c.F3[2], c.u3[2], fmaf(c.F3[0], c.u3[0], x64::fmul(c.F3[1], c.u3[1]))) * (1.0f / 3.0f) : 0.0f;
    const float Sr = S * rho;
 #pragma unroll
    for (int k = 0; k < 4; k++) {
@@ -186,7 +190,6 @@ __device__ __forceinline__ void shifted_pair(const ShiftedCell& c, float Gs, flo
    constexpr int cls = lat_norm2(Q, s);
    const float cu = cdot_f<Q, s>(c.u3);
    const float A = fmaf(c.wSr[cls], 0.5f * fmaf(cu, cu, -c.uu), c.wSd[cls]);
-   const float B = c.wSr[cls] * cu;
    float fs = 0.0f, fo = 0.0f;
    if (FORCE) {
       constexpr float w = (float)lat_w(Q, s);
@@ -195,8 +198,8 @@ __device__ __forceinline__ void shifted_pair(const ShiftedCell& c, float Gs, flo
       fs = Som2 * w * (cf + sym);
       fo = Som2 * w * (sym - cf);
    }
-   os = fmaf(om1, Gs, fmaf(omega, A + B, fs));
-   oob = fmaf(om1, Gob, fmaf(omega, A - B, fo));
+   os = fmaf(om1, Gs, fmaf(omega, fmaf(c.wSr[cls], cu, A), fs));
+   oob = fmaf(om1, Gob, fmaf(omega, fmaf(-c.wSr[cls], cu, A), fo));
 }
 
 // Output of the rest direction: A = w (S drho + S rho (-uu/2)), forcing -wf fu.
@@ -240,37 +243,111 @@ __device__ __forceinline__ void collide_f32(const float (&G)[Q], float (&o)[Q], 
    }
 }
 
-// Two cells (inputs G0, G1) with a uniform force: each direction's pair of
-// outputs goes to emit(s, o0, o1) as soon as it is made, so no output array
-// stays in registers.  The arithmetic per cell is collide_f32's.
-template <int Q, int ST, bool FORCE, int P = 0, class Emit2>
-__device__ __forceinline__ void collide2_pairs_f32(const float (&G0)[Q], const float (&G1)[Q], const ShiftedCell& c0,
-                                                   const ShiftedCell& c1, float om1, float omega, float Som2,
-                                                   Emit2& emit)
+// ------------------------------------- two cells in the packed halves
+// The arithmetic of collide_f32 for two cells with a uniform force, operation for
+// operation: inputs G[s] = (cell 0, cell 1); each direction's two outputs go to
+// emit(s, (o0, o1)) as soon as they are made, so no output array stays in
+// registers.
+struct ShiftedCell2 {
+   x64::f2 u3[3], fu, uu, wSd[4], wSr[4];
+   float F3[3];
+};
+
+template <int Q, int S_>
+__device__ __forceinline__ x64::f2 cdot_f2(const x64::f2 (&v)[3])
 {
+   constexpr int c0 = lat_c(Q, S_, 0), c1 = lat_c(Q, S_, 1), c2 = lat_c(Q, S_, 2);
+   x64::f2 r = {0.0f, 0.0f};
+   bool any = false;
+   if (c0 != 0) { r = c0 > 0 ? v[0] : x64::neg2(v[0]); any = true; }
+   if (c1 != 0) { r = any ? (c1 > 0 ? x64::add2(r, v[1]) : x64::sub2(r, v[1])) : (c1 > 0 ? v[1] : x64::neg2(v[1])); any = true; }
+   if (c2 != 0) { r = any ? (c2 > 0 ? x64::add2(r, v[2]) : x64::sub2(r, v[2])) : (c2 > 0 ? v[2] : x64::neg2(v[2])); }
+   return r;
+}
+
+template <int Q, int ST, bool FORCE>
+__device__ __forceinline__ ShiftedCell2 shifted_cell2(const x64::f2 (&G)[Q], const KParams& p)
+{
+   using namespace x64;
+   constexpr float S = ShiftScale<ST>::S;
+   constexpr float iS = 1.0f / S;
+   ShiftedCell2 c;
+   f2 Sd = {0.f, 0.f}, j[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll
+   for (int s = 0; s < Q; s++) {
+      Sd = add2(Sd, G[s]);
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+         if (lat_c(Q, s, d) > 0) j[d] = add2(j[d], G[s]);
+         if (lat_c(Q, s, d) < 0) j[d] = sub2(j[d], G[s]);
+      }
+   }
+   const f2 rho = fma2(Sd, dup2(iS), dup2(1.0f));
+   const f2 ir3 = {3.0f * __frcp_rn(rho.x), 3.0f * __frcp_rn(rho.y)};
+#pragma unroll
+   for (int d = 0; d < 3; d++) c.u3[d] = mul2(fma2(j[d], dup2(iS), dup2(FORCE ? 0.5f * p.Ff[d] : 0.0f)), ir3);
+   const f2 third = dup2(1.0f / 3.0f);
+   c.uu = mul2(fma2(c.u3[2], c.u3[2], fma2(c.u3[0], c.u3[0], mul2(c.u3[1], c.u3[1]))), third);
+   c.fu = {0.f, 0.f};
+   if constexpr (FORCE) {
+#pragma unroll
+      for (int d = 0; d < 3; d++) c.F3[d] = 3.0f * p.Ff[d];
+      c.fu = mul2(fma2(dup2(c.F3[2]), c.u3[2], fma2(dup2(c.F3[0]), c.u3[0], mul2(dup2(c.F3[1]), c.u3[1]))), third);
+   }
+   const f2 Sr = mul2(dup2(S), rho);
+#pragma unroll
+   for (int k = 0; k < 4; k++) {
+      float w;
+      if (Q == 19) w = k == 0 ? (float)(1.0 / 3.0) : (k == 1 ? (float)(1.0 / 18.0) : (float)(1.0 / 36.0));
+      else w = k == 0 ? (float)(8.0 / 27.0) : (k == 1 ? (float)(2.0 / 27.0) : (k == 2 ? (float)(1.0 / 54.0) : (float)(1.0 / 216.0)));
+      c.wSd[k] = mul2(dup2(w), Sd);
+      c.wSr[k] = mul2(dup2(w), Sr);
+   }
+   return c;
+}
+
+template <int Q, int ST, bool FORCE, int P = 0, class Emit2>
+__device__ __forceinline__ void shifted_pairs2(const x64::f2 (&G)[Q], const ShiftedCell2& c, const KParams& p, float Som2,
+                                               Emit2& emit)
+{
+   using namespace x64;
    if constexpr (P < (Q - 1) / 2) {
       constexpr int s = pair_rep<Q, P>();
       constexpr int ob = lat_opp(Q, s);
-      float a0, b0, a1, b1;
-      shifted_pair<Q, ST, FORCE, P>(c0, G0[s], G0[ob], om1, omega, Som2, a0, b0);
-      shifted_pair<Q, ST, FORCE, P>(c1, G1[s], G1[ob], om1, omega, Som2, a1, b1);
-      emit(s, a0, a1);
-      emit(ob, b0, b1);
-      collide2_pairs_f32<Q, ST, FORCE, P + 1>(G0, G1, c0, c1, om1, omega, Som2, emit);
+      constexpr int cls = lat_norm2(Q, s);
+      const f2 cu = cdot_f2<Q, s>(c.u3);
+      const f2 A = fma2(c.wSr[cls], mul2(dup2(0.5f), fma2(cu, cu, neg2(c.uu))), c.wSd[cls]);
+      f2 fs = {0.f, 0.f}, fo = {0.f, 0.f};
+      if constexpr (FORCE) {
+         constexpr float w = (float)lat_w(Q, s);
+         const f2 cf = dup2(cdot_f<Q, s>(c.F3));
+         const f2 sym = fma2(cu, cf, neg2(c.fu));
+         const f2 Sw = dup2(Som2 * w);
+         fs = mul2(Sw, add2(cf, sym));
+         fo = mul2(Sw, sub2(sym, cf));
+      }
+      const f2 om1 = dup2(p.om1f), om = dup2(p.omegaf);
+      emit(s, fma2(om1, G[s], fma2(om, fma2(c.wSr[cls], cu, A), fs)));
+      emit(ob, fma2(om1, G[ob], fma2(om, fma2(neg2(c.wSr[cls]), cu, A), fo)));
+      shifted_pairs2<Q, ST, FORCE, P + 1>(G, c, p, Som2, emit);
    }
 }
 
 template <int Q, int ST, bool FORCE, class Emit2>
-__device__ __forceinline__ void collide2_f32_emit(const float (&G0)[Q], const float (&G1)[Q], const KParams& p,
-                                                  Emit2& emit)
+__device__ __forceinline__ void collide2_f32_emit(const x64::f2 (&G)[Q], const KParams& p, Emit2& emit)
 {
-   const float F0 = FORCE ? p.Ff[0] : 0.0f, F1 = FORCE ? p.Ff[1] : 0.0f, F2 = FORCE ? p.Ff[2] : 0.0f;
-   const ShiftedCell c0 = shifted_cell<Q, ST, FORCE>(G0, F0, F1, F2);
-   const ShiftedCell c1 = shifted_cell<Q, ST, FORCE>(G1, F0, F1, F2);
+   using namespace x64;
+   const ShiftedCell2 c = shifted_cell2<Q, ST, FORCE>(G, p);
    const float Som2 = ShiftScale<ST>::S * p.om2f;
-   collide2_pairs_f32<Q, ST, FORCE>(G0, G1, c0, c1, p.om1f, p.omegaf, Som2, emit);
+   shifted_pairs2<Q, ST, FORCE>(G, c, p, Som2, emit);
    constexpr int R = lat_rest(Q);
-   emit(R, shifted_rest<Q, ST, FORCE>(c0, G0[R], p, Som2), shifted_rest<Q, ST, FORCE>(c1, G1[R], p, Som2));
+   const f2 A = fma2(c.wSr[0], mul2(dup2(-0.5f), c.uu), c.wSd[0]);
+   f2 fr = {0.f, 0.f};
+   if constexpr (FORCE) {
+      const float wf = (Q == 19 && p.compat) ? (float)(1.0 / 36.0) : (float)lat_w(Q, R);
+      fr = mul2(dup2(-Som2 * wf), c.fu);
+   }
+   emit(R, fma2(dup2(p.om1f), G[R], fma2(dup2(p.omegaf), A, fr)));
 }
 
 }  // namespace lbm

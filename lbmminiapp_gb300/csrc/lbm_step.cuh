@@ -139,7 +139,7 @@ __device__ __forceinline__ void cell_force_f32(const KParams& p, int64_t c, floa
 // One launch = one time step (or one range of it) of one propagation kind.  The
 // exact FP64 arithmetic needs 16 warps per SM to keep its two pipes busy.
 template <int Q, int ST, int AR, int KIND, bool LINKS, bool FIELDS, typename IT>
-__global__ void __launch_bounds__(256, AR == AR_F64 ? 2 : 1) step_kernel(const KParams p, const typename Store<ST>::T* src,
+__global__ void __launch_bounds__(256, AR == AR_F64 ? 2 : 0) step_kernel(const KParams p, const typename Store<ST>::T* src,
                                                    typename Store<ST>::T* dst)
 {
    wait_prior_grid();
@@ -240,6 +240,14 @@ __device__ constexpr bool write_shifted_x(int s)
 template <int Q, int ST>
 constexpr int pair_min_blocks() { return Q == 27 ? 2 : (Store<ST>::bytes == 2 ? 4 : 3); }
 
+// Whether the two cells collide in the packed instructions' halves.  At 256^3 that
+// takes the FP16 steps (even / odd / push / pull) from 329 / 407 / 368 / 334 to
+// 312 / 372 / 346 / 330 us for D3Q27, from 199 / - / 226 / 214 to 195 / - / 206 /
+// 215 us for D3Q19.  The D3Q19 AA odd step, which has neighbour addresses for its
+// reads and its writes, spills with it (244 -> 273 us), so its cells stay apart.
+template <int Q, int KIND>
+constexpr bool pair_packed() { return !(Q == 19 && KIND == K_AA_ODD); }
+
 template <int Q, int ST, int KIND, typename IT>
 __global__ void __launch_bounds__(256, pair_min_blocks<Q, ST>()) step_pair_kernel(const KParams p, const typename Store<ST>::T* src,
                                                         typename Store<ST>::T* dst)
@@ -258,37 +266,47 @@ __global__ void __launch_bounds__(256, pair_min_blocks<Q, ST>()) step_pair_kerne
    const T* s1 = src + c1.c;
    T* d0 = dst + c0.c;
    T* d1 = dst + c1.c;
-   float g0[Q], g1[Q], o0[Q], o1[Q];
+   x64::f2 g[Q];
 #pragma unroll
    for (int s = 0; s < Q; s++) {
       const Access a0 = read_access<Q, KIND, false>(c0, 0u, s);
       if (read_shifted_x<Q, KIND>(s)) {
          const Access a1 = read_access<Q, KIND, false>(c1, 0u, s);
-         g0[s] = load_raw(slot_ptr(s0, pb, a0));
-         g1[s] = load_raw(slot_ptr(s1, pb, a1));
+         g[s] = {load_raw(slot_ptr(s0, pb, a0)), load_raw(slot_ptr(s1, pb, a1))};
       } else {
          const float2 v = PV::get(*reinterpret_cast<const typename PV::V*>(slot_ptr(s0, pb, a0)));
-         g0[s] = v.x;
-         g1[s] = v.y;
+         g[s] = {v.x, v.y};
       }
    }
-   if (p.forced) {
-      collide_f32<Q, ST, true>(g0, o0, p.Ff[0], p.Ff[1], p.Ff[2], 0.0f, p);
-      collide_f32<Q, ST, true>(g1, o1, p.Ff[0], p.Ff[1], p.Ff[2], 0.0f, p);
-   } else {
-      collide_f32<Q, ST, false>(g0, o0, 0.0f, 0.0f, 0.0f, 0.0f, p);
-      collide_f32<Q, ST, false>(g1, o1, 0.0f, 0.0f, 0.0f, 0.0f, p);
-   }
-#pragma unroll
-   for (int s = 0; s < Q; s++) {
+   auto emit = [&](int s, x64::f2 o) {
       const Access a0 = write_access<Q, KIND, false>(c0, 0u, s);
       if (write_shifted_x<Q, KIND>(s)) {
          const Access a1 = write_access<Q, KIND, false>(c1, 0u, s);
-         store_raw(slot_ptr(d0, pb, a0), o0[s]);
-         store_raw(slot_ptr(d1, pb, a1), o1[s]);
+         store_raw(slot_ptr(d0, pb, a0), o.x);
+         store_raw(slot_ptr(d1, pb, a1), o.y);
       } else {
-         *reinterpret_cast<typename PV::V*>(slot_ptr(d0, pb, a0)) = PV::put(o0[s], o1[s]);
+         *reinterpret_cast<typename PV::V*>(slot_ptr(d0, pb, a0)) = PV::put(o.x, o.y);
       }
+   };
+   if constexpr (pair_packed<Q, KIND>()) {
+      if (p.forced) collide2_f32_emit<Q, ST, true>(g, p, emit);
+      else collide2_f32_emit<Q, ST, false>(g, p, emit);
+   } else {
+      float g0[Q], g1[Q], o0[Q], o1[Q];
+#pragma unroll
+      for (int s = 0; s < Q; s++) {
+         g0[s] = g[s].x;
+         g1[s] = g[s].y;
+      }
+      if (p.forced) {
+         collide_f32<Q, ST, true>(g0, o0, p.Ff[0], p.Ff[1], p.Ff[2], 0.0f, p);
+         collide_f32<Q, ST, true>(g1, o1, p.Ff[0], p.Ff[1], p.Ff[2], 0.0f, p);
+      } else {
+         collide_f32<Q, ST, false>(g0, o0, 0.0f, 0.0f, 0.0f, 0.0f, p);
+         collide_f32<Q, ST, false>(g1, o1, 0.0f, 0.0f, 0.0f, 0.0f, p);
+      }
+#pragma unroll
+      for (int s = 0; s < Q; s++) emit(s, {o0[s], o1[s]});
    }
 }
 
