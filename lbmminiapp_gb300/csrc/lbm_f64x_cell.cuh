@@ -27,21 +27,25 @@ __device__ __forceinline__ void collide_f64x(uint64_t (&bits)[Q], const KParams&
 }
 
 // Input pattern s read again from shared memory (direction s at byte 256 s
-// from the lane's first), raw or split into a float pair.  The load is
-// volatile so that the compiler does not keep the first load's value live in
-// registers instead.
+// from the lane's first).  The load is volatile so that the compiler does not
+// keep the first load's value live in registers instead.  REST: the rest
+// population is in a register.
+template <int Q, bool REST>
 struct AgainFromShared {
    static constexpr bool kRefetch = true;
    uint32_t addr;
+   uint64_t rest;
    __device__ __forceinline__ uint64_t raw(int s) const
    {
+      if (REST && s == lat_rest(Q)) return rest;
       unsigned long long v;
       asm volatile("ld.shared.u64 %0, [%1];\n" : "=l"(v) : "r"(addr + 256u * (uint32_t)s));
       return v;
    }
 };
 
-// collide_f64x for inputs that stay in shared memory (direction s at in[32 s]),
+// collide_f64x for inputs that stay in shared memory (direction s at in[32 s]; with
+// REST the last one, the rest direction, is `rest`),
 // with each output handed to emit(s, pattern) as it is made, so neither the
 // input nor the output patterns stay in registers through the fast path: the
 // moment sums read the inputs once, the update reads them again.  If
@@ -54,14 +58,15 @@ struct AgainFromShared {
 // all four forms' code allocates registers for the worst of them (D3Q19 AA odd
 // step, 256x128x128: 219 us against 211).  kForceOther holds forms 1 and 2.
 constexpr int kForceOther = 1;
-template <int Q, int FORCE, class Emit>
-__device__ __forceinline__ void collide_f64x_shared_emit(const unsigned long long* in, const KParams& p, Emit& emit)
+template <int Q, int FORCE, bool REST, class Emit>
+__device__ __forceinline__ void collide_f64x_shared_emit(const unsigned long long* in, uint64_t rest, const KParams& p,
+                                                         Emit& emit)
 {
    uint64_t bits[Q];
 #pragma unroll
-   for (int s = 0; s < Q; s++) bits[s] = in[s * 32];
+   for (int s = 0; s < Q; s++) bits[s] = REST && s == lat_rest(Q) ? rest : in[s * 32];
    const x64::Consts k = collide_consts<Q>(p);
-   const AgainFromShared again{(uint32_t)__cvta_generic_to_shared(in)};
+   const AgainFromShared<Q, REST> again{(uint32_t)__cvta_generic_to_shared(in), rest};
    bool fast;
    if constexpr (FORCE == kForceOther)
       fast = p.forced == 2 ? collide_f64x_fast_emit<Q, 2>(bits, k, p.compat, emit, again)

@@ -124,13 +124,15 @@ __global__ void __launch_bounds__(kSparseThreads, sparse_min_blocks<Q>()) sparse
 // and each output is stored as the collision makes it.  AA stays race-free
 // under the prefetch: a fluid point's read and write locations are the same
 // set, disjoint from every other point's.
-// Warps per block and blocks per SM: 12 warps at up to 168 registers, D3Q27 in
-// one block so that their shared memory fits the 164 KB carve-out
-// (lbm_step_async.cuh says why that matters).
+// Warps per block and blocks per SM: 12 warps at up to 168 registers, whose shared
+// memory fits the 164 KB carve-out (lbm_step_async.cuh says why that matters).
 template <int Q>
-constexpr int sparse_warps() { return Q == 19 ? 4 : 12; }
+constexpr int sparse_warps() { return 4; }
 template <int Q>
-constexpr int sparse_blocks() { return Q == 19 ? 3 : 1; }
+constexpr int sparse_blocks() { return 3; }
+// The D3Q27 rest population in a register, as there.
+template <int Q>
+constexpr bool sparse_rest() { return Q == 27; }
 
 template <int KIND>
 constexpr bool sparse_gathers() { return KIND == K_AA_ODD || KIND == K_AB_PULL; }
@@ -157,12 +159,14 @@ __global__ void __launch_bounds__(sparse_warps<Q>() * 32, sparse_blocks<Q>()) sp
    extern __shared__ __align__(16) unsigned long long sparse_smem[];
    const int lane = threadIdx.x & 31;
    const int warp = threadIdx.x >> 5;
-   constexpr int kWarps = sparse_warps<Q>();
+   const uint32_t kWarps = blockDim.x >> 5;
    const uint32_t nw = gridDim.x * kWarps;
    wait_prior_grid();
-   unsigned long long* mine = sparse_smem + (size_t)warp * kAsyncStages * Q * 32;
+   constexpr bool kRest = sparse_rest<Q>();
+   constexpr int kRows = kRest ? Q - 1 : Q;   // directions staged per tile
+   unsigned long long* mine = sparse_smem + (size_t)warp * kAsyncStages * kRows * 32;
    const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(mine);
-   constexpr uint32_t kStageBytes = Q * 32 * 8;
+   constexpr uint32_t kStageBytes = kRows * 32 * 8;
    const unsigned long long* s64 = reinterpret_cast<const unsigned long long*>(src);
    // fluid index of this lane in tile tt, and whether it is inside the range
    auto point = [&](uint32_t tt, bool& act) {
@@ -177,12 +181,14 @@ __global__ void __launch_bounds__(sparse_warps<Q>() * 32, sparse_blocks<Q>()) sp
 #pragma unroll
       for (int s = 0; s < Q; s++) ahead[s] = act ? (uint32_t)__ldg(adj + (size_t)nf * s + i) : 0u;
    };
-   auto issue = [&](uint32_t tt, uint32_t sb) {
+   uint64_t rest = 0, rest_next = 0;
+   auto issue = [&](uint32_t tt, uint32_t sb, uint64_t& r0) {
       bool act;
       const uint32_t i = point(tt, act);
       if (!act) return;
+      if constexpr (kRest) r0 = s64[sparse_gathers<KIND>() ? ahead[Q - 1] : nf * (uint32_t)(Q - 1) + i];
 #pragma unroll
-      for (int s = 0; s < Q; s++) {
+      for (int s = 0; s < kRows; s++) {
          uint32_t r;
          if (KIND == K_AA_EVEN) r = nf * (uint32_t)lat_opp(Q, s) + i;
          else if (KIND == K_AB_PUSH) r = nf * (uint32_t)s + i;
@@ -203,13 +209,13 @@ __global__ void __launch_bounds__(sparse_warps<Q>() * 32, sparse_blocks<Q>()) sp
       uint32_t t1 = t + nw < ntiles ? t + nw : ntiles;
       uint32_t t2 = t + 2u * nw < ntiles ? t + 2u * nw : ntiles;
       if (sparse_gathers<KIND>()) load_ahead(t);
-      issue(t, sbase);
+      issue(t, sbase, rest);
       cp_async_commit();
       if (sparse_gathers<KIND>() && t1 < ntiles) load_ahead(t1);
       int stage = 0;
       for (;;) {
          if (t1 < ntiles) {
-            issue(t1, sbase + (stage ^ 1) * kStageBytes);
+            issue(t1, sbase + (stage ^ 1) * kStageBytes, rest_next);
             if (sparse_gathers<KIND>() && t2 < ntiles) load_ahead(t2);
          }
          cp_async_commit();
@@ -226,12 +232,13 @@ __global__ void __launch_bounds__(sparse_warps<Q>() * 32, sparse_blocks<Q>()) sp
                }
             }
             const SparseEmit<Q, KIND> emit{dst, nf, i, wl};
-            collide_f64x_shared_emit<Q, FORCE>(mine + stage * Q * 32 + lane, p, emit);
+            collide_f64x_shared_emit<Q, FORCE, kRest>(mine + stage * kRows * 32 + lane, rest, p, emit);
          }
          if (t1 >= ntiles) break;
          t = t1;
          t1 = t2;
          t2 = feed_after(feed, fed, t2, p.sched, 3u * nw, ntiles, nw, lane);
+         rest = rest_next;
          stage ^= 1;
       }
    }
@@ -250,7 +257,7 @@ cudaError_t launch_sparse_async_form(const KParams& p, const int32_t* adj, int64
    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
    constexpr int kWarps = sparse_warps<Q>(), kBlocks = sparse_blocks<Q>();
    auto kern = sparse_async_kernel<Q, KIND, FORCE>;
-   constexpr size_t smem = (size_t)kWarps * kAsyncStages * Q * 32 * sizeof(unsigned long long);
+   constexpr size_t smem = (size_t)kWarps * kAsyncStages * (sparse_rest<Q>() ? Q - 1 : Q) * 32 * sizeof(unsigned long long);
    int cached = grid_of_device[dev].load(std::memory_order_relaxed);
    if (cached == 0) {
       e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -262,15 +269,14 @@ cudaError_t launch_sparse_async_form(const KParams& p, const int32_t* adj, int64
       if (e != cudaSuccess) return e;
       e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
       if (e != cudaSuccess) return e;
-      if (per_sm < 1) return cudaErrorInvalidConfiguration;
-      cached = (per_sm < kBlocks ? per_sm : kBlocks) * nsm;
+      if (per_sm < kBlocks) return cudaErrorInvalidConfiguration;
+      cached = kBlocks * nsm;   // no more than the carve-out is meant for
       grid_of_device[dev].store(cached, std::memory_order_relaxed);
    }
    const uint32_t ntiles = (uint32_t)((count + 31) / 32);
-   const uint32_t need = (ntiles + kWarps - 1) / kWarps;
-   const unsigned grid = (unsigned)(need < (uint32_t)cached ? need : (uint32_t)cached);
-   return launch_overlapped(kern, dim3(grid), dim3(kWarps * 32), smem, stream, p, adj, (uint32_t)nfluid,
-                            (uint32_t)start, (uint32_t)count, ntiles, src, dst);
+   const AsyncLaunch L = async_launch(ntiles, (uint32_t)cached / kBlocks, kBlocks, kWarps);
+   return launch_overlapped(kern, dim3(L.blocks), dim3(L.warps * 32), smem / kWarps * L.warps, stream, p, adj,
+                            (uint32_t)nfluid, (uint32_t)start, (uint32_t)count, ntiles, src, dst);
 }
 
 template <int Q, int KIND>

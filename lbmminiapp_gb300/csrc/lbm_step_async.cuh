@@ -33,13 +33,25 @@ namespace lbm {
 //   D3Q19 AA even / odd step   197 / 211 us,  -,               246 / 293 us
 //   D3Q27 AA even / odd step   283 / 342 us,  295 / 356 us,    362 / 438 us
 //   D3Q27 AB push / pull step  302 / 309 us,  316 / 305 us,    375 / 395 us
-// So D3Q19 runs 16 warps in two blocks (128 registers), D3Q27 12 warps in one
-// (168 registers; as three blocks the 1 KB that each reserves would take them
-// over 164 KB, and 16 warps need 228 KB), and the launch asks for the carve-out.
-template <int Q>
-constexpr int async_warps() { return Q == 19 ? 8 : 12; }
-template <int Q>
-constexpr int async_min_blocks() { return Q == 19 ? 2 : 1; }
+// So D3Q19 runs 16 warps in two blocks (128 registers) and D3Q27 12 warps (168
+// registers; 16 warps need 228 KB), and the launch asks for the carve-out.  The
+// 12 warps come in two forms:
+//   REST   three blocks, with the rest population, which every kind reads from the
+//          own cell, in a register (as three blocks with all 27 staged they take
+//          165 KB): odd 324 us, pull 295 us, even 291 us, push 303 us (links 317);
+//   else   one block, all directions staged: odd 342, pull 309, even 281, push
+//          302 us (links 308).
+// The gathers run the first; the others the second, but the first for grids of
+// fewer than 16 tiles per warp, where a step overlaps the next by the block (48^3:
+// AA 11.5 us a step against 13.6, push 11.6 against 13.7).  D3Q19 with a rest
+// register: 201 / 219 us, so not there.
+template <int Q, bool REST>
+constexpr int async_warps() { return Q == 19 ? 8 : (REST ? 4 : 12); }
+template <int Q, bool REST>
+constexpr int async_min_blocks() { return Q == 19 ? 2 : (REST ? 3 : 1); }
+// Directions staged in shared memory per tile.
+template <int Q, bool REST>
+constexpr int async_rows() { return REST ? Q - 1 : Q; }
 constexpr int kAsyncStages = 2;
 constexpr int kBlockReserve = 1024;          // shared memory the system takes per block
 constexpr int kMaxSharedPerSM = 228 * 1024;
@@ -50,10 +62,10 @@ constexpr int carveout_percent(int blocks, size_t smem)
    return (int)((blocks * (smem + kBlockReserve) * 100 + kMaxSharedPerSM - 1) / kMaxSharedPerSM);
 }
 
-template <int Q>
+template <int Q, bool REST>
 constexpr size_t async_smem_bytes()
 {
-   return (size_t)async_warps<Q>() * kAsyncStages * Q * 32 * sizeof(unsigned long long);
+   return (size_t)async_warps<Q, REST>() * kAsyncStages * async_rows<Q, REST>() * 32 * sizeof(unsigned long long);
 }
 
 // Tiles of 32 cells: tile t covers x in [32 (t mod ntx), +32) of row t / ntx,
@@ -144,25 +156,27 @@ __device__ __forceinline__ bool tile_linked(uint32_t lk)
    return __any_sync(0xFFFFFFFFu, (lk & ~kSolidBit) != 0u);
 }
 
-template <int Q, int KIND, bool LINKS>
+template <int Q, int KIND, bool LINKS, bool REST>
 __device__ __forceinline__ void async_issue_cell(const PlanePtrs& pp, const TileLane& tl, int lane, uint32_t sbuf)
 {
    const uint32_t c = (uint32_t)tl.ci.c;
 #pragma unroll
-   for (int s = 0; s < Q; s++) {
+   for (int s = 0; s < async_rows<Q, REST>(); s++) {
       const Access a = read_access<Q, KIND, LINKS>(tl.ci, tl.lk, s);
       cp_async8(sbuf + (uint32_t)(s * 32 + lane) * 8u, pp.src[a.slot] + (c + (uint32_t)a.off));
    }
 }
 
-template <int Q, int KIND, bool LINKS, bool RAGGED>
-__device__ __forceinline__ void async_issue(const PlanePtrs& pp, const TileLane& tl, int lane, uint32_t sbuf)
+// The copies of a tile's populations (REST: the rest one into a register).
+template <int Q, int KIND, bool LINKS, bool RAGGED, bool REST>
+__device__ __forceinline__ void async_issue(const PlanePtrs& pp, const TileLane& tl, int lane, uint32_t sbuf, uint64_t& rest)
 {
    constexpr bool kGathers = KIND == K_AA_ODD || KIND == K_AB_PULL;
    const bool linked = LINKS && kGathers && tile_linked(tl.lk);
    if ((LINKS || RAGGED) && !tl.active) return;
-   if (LINKS && kGathers && linked) async_issue_cell<Q, KIND, LINKS>(pp, tl, lane, sbuf);
-   else async_issue_cell<Q, KIND, false>(pp, tl, lane, sbuf);
+   if constexpr (REST) rest = pp.src[lat_rest(Q)][(uint32_t)tl.ci.c];
+   if (LINKS && kGathers && linked) async_issue_cell<Q, KIND, LINKS, REST>(pp, tl, lane, sbuf);
+   else async_issue_cell<Q, KIND, false, REST>(pp, tl, lane, sbuf);
 }
 
 // Stores each output straight to its target slot.  AA stays race-free with
@@ -180,20 +194,21 @@ struct StoreEmit {
    }
 };
 
-template <int Q, int KIND, bool LINKS, bool RAGGED, int FORCE>
-__global__ void __launch_bounds__(async_warps<Q>() * 32, async_min_blocks<Q>()) step_async_kernel(const KParams p, const AsyncGeom ag,
+template <int Q, int KIND, bool LINKS, bool RAGGED, int FORCE, bool REST>
+__global__ void __launch_bounds__(async_warps<Q, REST>() * 32, async_min_blocks<Q, REST>()) step_async_kernel(const KParams p, const AsyncGeom ag,
                                                                       const PlanePtrs pp)
 {
    extern __shared__ __align__(16) unsigned long long async_smem[];
    const int lane = threadIdx.x & 31;
    const int warp = threadIdx.x >> 5;
-   constexpr int kWarps = async_warps<Q>();
+   const uint32_t kWarps = blockDim.x >> 5;
    const uint32_t nw = gridDim.x * kWarps;
    const uint32_t ntiles = ag.ntiles;
    wait_prior_grid();
-   unsigned long long* mine = async_smem + (size_t)warp * kAsyncStages * Q * 32;
+   constexpr int kRows = async_rows<Q, REST>();
+   unsigned long long* mine = async_smem + (size_t)warp * kAsyncStages * kRows * 32;
    const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(mine);
-   constexpr uint32_t kStageBytes = Q * 32 * 8;
+   constexpr uint32_t kStageBytes = kRows * 32 * 8;
    // tiles: three per warp in a fixed order, then the launch's tile feed (8
    // counters for the D3Q19 tiles, which it hands out fastest); t is collided
    // while t1's populations are in flight and t2's link words are loaded
@@ -207,7 +222,8 @@ __global__ void __launch_bounds__(async_warps<Q>() * 32, async_min_blocks<Q>()) 
       TileLane cur;
       tile_lane<LINKS, RAGGED>(p, ag, t, lane, LINKS ? tile_link(p, ag, t, lane) : 0u, cur);
       uint32_t lk_ahead = (LINKS && t1 < ntiles) ? tile_link(p, ag, t1, lane) : 0u;
-      async_issue<Q, KIND, LINKS, RAGGED>(pp, cur, lane, sbase);
+      uint64_t rest = 0, rest_next = 0;
+      async_issue<Q, KIND, LINKS, RAGGED, REST>(pp, cur, lane, sbase, rest);
       cp_async_commit();
       int stage = 0;
       for (;;) {
@@ -215,7 +231,7 @@ __global__ void __launch_bounds__(async_warps<Q>() * 32, async_min_blocks<Q>()) 
          if (t1 < ntiles) {
             tile_lane<LINKS, RAGGED>(p, ag, t1, lane, lk_ahead, nxt);
             if (LINKS && t2 < ntiles) lk_ahead = tile_link(p, ag, t2, lane);
-            async_issue<Q, KIND, LINKS, RAGGED>(pp, nxt, lane, sbase + (stage ^ 1) * kStageBytes);
+            async_issue<Q, KIND, LINKS, RAGGED, REST>(pp, nxt, lane, sbase + (stage ^ 1) * kStageBytes, rest_next);
          }
          cp_async_commit();
          cp_async_wait_prev();
@@ -223,15 +239,15 @@ __global__ void __launch_bounds__(async_warps<Q>() * 32, async_min_blocks<Q>()) 
          // re-reads its inputs from shared memory: neither the Q input nor the
          // Q output patterns stay in registers
          constexpr bool kScatters = KIND == K_AA_ODD || KIND == K_AB_PUSH;
-         const unsigned long long* in = mine + stage * Q * 32 + lane;
+         const unsigned long long* in = mine + stage * kRows * 32 + lane;
          const bool linked = LINKS && kScatters && tile_linked(cur.lk);
          if (!(LINKS || RAGGED) || cur.active) {
             if (LINKS && kScatters && linked) {
                StoreEmit<Q, KIND, LINKS> emit{pp, cur.ci, cur.lk};
-               collide_f64x_shared_emit<Q, FORCE>(in, p, emit);
+               collide_f64x_shared_emit<Q, FORCE, REST>(in, rest, p, emit);
             } else {
                StoreEmit<Q, KIND, false> emit{pp, cur.ci, 0u};
-               collide_f64x_shared_emit<Q, FORCE>(in, p, emit);
+               collide_f64x_shared_emit<Q, FORCE, REST>(in, rest, p, emit);
             }
          }
          if (t1 >= ntiles) break;
@@ -239,6 +255,7 @@ __global__ void __launch_bounds__(async_warps<Q>() * 32, async_min_blocks<Q>()) 
          t1 = t2;
          t2 = feed_after(feed, fed, t2, p.sched, 3u * nw, ntiles, nw, lane);
          cur = nxt;
+         rest = rest_next;
          stage ^= 1;
       }
    }
@@ -255,10 +272,26 @@ inline AsyncGeom async_geom(int nx, int ny, int nz)
    return g;
 }
 
+// Blocks and warps per block of a launch on nsm SMs, per_sm blocks of max_warps on
+// each at most.  A grid with fewer tiles than that many warps runs smaller blocks
+// on as many SMs, not full blocks on a few (D3Q27 AB pull, 24x21x38: 798 tiles, 67
+// blocks of 12 warps left 85 of the 152 SMs idle: 5.5 us, 4.2 us spread).
+struct AsyncLaunch {
+   unsigned blocks, warps;
+};
+inline AsyncLaunch async_launch(uint32_t ntiles, uint32_t nsm, uint32_t per_sm, uint32_t max_warps)
+{
+   const uint32_t each = (ntiles + nsm - 1) / nsm;
+   const uint32_t w = each < max_warps ? (each ? each : 1u) : max_warps;
+   const uint32_t need = (ntiles + w - 1) / w;
+   const uint32_t resident = nsm * per_sm;
+   return {need < resident ? need : resident, w};
+}
+
 // Persistent grid: as many blocks as fit on the device at once (queried once
 // per device and kernel; the shared-memory opt-in is set at the same time).
-template <int Q, int KIND, bool LINKS, bool RAGGED, int FORCE>
-cudaError_t launch_async_form(const KParams& p, const AsyncGeom& ag, const void* src, void* dst, cudaStream_t stream)
+template <int Q, int KIND, bool LINKS, bool RAGGED, int FORCE, bool REST>
+cudaError_t launch_async_kernel(const KParams& p, const AsyncGeom& ag, const void* src, void* dst, cudaStream_t stream)
 {
    // Persistent grid size per device ordinal, set once (the value is the same
    // whichever thread computes it first).
@@ -267,35 +300,55 @@ cudaError_t launch_async_form(const KParams& p, const AsyncGeom& ag, const void*
    cudaError_t e = cudaGetDevice(&dev);
    if (e != cudaSuccess) return e;
    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-   auto kern = step_async_kernel<Q, KIND, LINKS, RAGGED, FORCE>;
-   constexpr int kWarps = async_warps<Q>();
-   constexpr size_t smem = async_smem_bytes<Q>();
+   auto kern = step_async_kernel<Q, KIND, LINKS, RAGGED, FORCE, REST>;
+   constexpr int kWarps = async_warps<Q, REST>();
+   constexpr size_t smem = async_smem_bytes<Q, REST>();
    int cached = grid_of_device[dev].load(std::memory_order_relaxed);
    if (cached == 0) {
       e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
       e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
-                               carveout_percent(async_min_blocks<Q>(), smem));
+                               carveout_percent(async_min_blocks<Q, REST>(), smem));
       if (e != cudaSuccess) return e;
       int per_sm = 0, nsm = 0;
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kWarps * 32, smem);
       if (e != cudaSuccess) return e;
       e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
       if (e != cudaSuccess) return e;
-      if (per_sm < 1) return cudaErrorInvalidConfiguration;
-      // no more than the carve-out is meant for
-      cached = (per_sm < async_min_blocks<Q>() ? per_sm : async_min_blocks<Q>()) * nsm;
+      if (per_sm < async_min_blocks<Q, REST>()) return cudaErrorInvalidConfiguration;
+      cached = async_min_blocks<Q, REST>() * nsm;   // no more than the carve-out is meant for
       grid_of_device[dev].store(cached, std::memory_order_relaxed);
    }
-   const uint32_t need = (ag.ntiles + kWarps - 1) / kWarps;
-   const unsigned grid = (unsigned)(need < (uint32_t)cached ? need : (uint32_t)cached);
+   const AsyncLaunch L = async_launch(ag.ntiles, (uint32_t)cached / async_min_blocks<Q, REST>(), async_min_blocks<Q, REST>(),
+                                      kWarps);
    PlanePtrs pp;
    for (int s = 0; s < 27; s++) {
       const int k = s < Q ? s : 0;
       pp.src[s] = static_cast<const unsigned long long*>(src) + (int64_t)k * p.plane;
       pp.dst[s] = static_cast<unsigned long long*>(dst) + (int64_t)k * p.plane;
    }
-   return launch_overlapped(kern, dim3(grid), dim3(kWarps * 32), smem, stream, p, ag, pp);
+   return launch_overlapped(kern, dim3(L.blocks), dim3(L.warps * 32), smem / kWarps * L.warps, stream, p, ag, pp);
+}
+
+// Rule for REST (at async_warps).
+template <int Q, int KIND, bool LINKS, bool RAGGED, int FORCE>
+cudaError_t launch_async_form(const KParams& p, const AsyncGeom& ag, const void* src, void* dst, cudaStream_t stream)
+{
+   if constexpr (Q == 27) {
+      constexpr bool kGathers = KIND == K_AA_ODD || KIND == K_AB_PULL;
+      if constexpr (kGathers || FORCE == kForceOther) {
+         return launch_async_kernel<Q, KIND, LINKS, RAGGED, FORCE, true>(p, ag, src, dst, stream);
+      } else {
+         int dev = 0, nsm = 0;
+         cudaError_t e = cudaGetDevice(&dev);
+         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+         if (e != cudaSuccess) return e;
+         if ((uint64_t)ag.ntiles < (uint64_t)kFeedMinTiles * 12u * (uint64_t)nsm)
+            return launch_async_kernel<Q, KIND, LINKS, RAGGED, FORCE, true>(p, ag, src, dst, stream);
+      }
+   }
+   if constexpr (Q == 19 || !(KIND == K_AA_ODD || KIND == K_AB_PULL || FORCE == kForceOther))
+      return launch_async_kernel<Q, KIND, LINKS, RAGGED, FORCE, false>(p, ag, src, dst, stream);
 }
 
 // links: the grid has link words.  Kernels exist for no force and the velocity
