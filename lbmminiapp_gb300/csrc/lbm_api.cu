@@ -1072,7 +1072,9 @@ lbm_status lbm_loss(lbm_handle* h, const void* state, int loss_kind, const doubl
    a.loss_kind = loss_kind;
    a.loss_weight = weight;
    a.time_weight = time_weight;
-   LBM_CUDA(h, launch_loss(h->Q, h->storage, a, h->partials, kReduceBlocks, h->reduce_out, h->stream));
+   // one cell per thread as far as the scratch goes (one double per block)
+   const int blocks = (int)std::min<int64_t>(4 * kReduceBlocks, (h->ncell + kReduceThreads - 1) / kReduceThreads);
+   LBM_CUDA(h, launch_loss(h->Q, h->storage, a, h->partials, blocks, h->reduce_out, h->stream));
    LBM_CUDA(h, cudaMemcpyAsync(out_host, h->reduce_out, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
    LBM_CUDA(h, cudaStreamSynchronize(h->stream));
    return LBM_OK;

@@ -40,9 +40,7 @@ cudaError_t launch_kind(const Launch& L, const KParams& p, const void* src, void
                                   s, d);
       }
       if (L.async_low && links && !fields) {
-         const bool ragged = p.nx % 32 != 0;
-         return ragged ? launch_async_low<Q, ST, KIND, true, true>(p, L.ag, src, dst, L.stream)
-                       : launch_async_low<Q, ST, KIND, true, false>(p, L.ag, src, dst, L.stream);
+         return launch_async_low<Q, ST, KIND>(p, L.ag, src, dst, L.stream);
       }
    }
    if constexpr (ST == ST_F64 && AR == AR_F64X) {

@@ -1,15 +1,14 @@
 // Software-pipelined step kernel for FP64 storage with F64X arithmetic (any
 // box; link words for walls and solids; no per-cell fields).
 //
-// The F64X collision is about 1.7k instructions per cell, so the plain
-// one-cell-per-thread kernel spends its time either issuing or waiting on its
-// 19/27 loads with only 16 warps per SM resident (128 registers per thread).
-// Here every warp is persistent and works on tiles of 32 consecutive cells of
-// one x row: while it collides tile k it already has the loads of tile k+1 in
-// flight as cp.async copies (8 bytes per thread and direction) into its own
-// two-stage shared-memory buffer, so the loads hold no registers and their
-// latency overlaps the collision.  Each thread reads back only what it copied
-// itself, so cp.async.wait_group is the only synchronisation needed.
+// The F64X collision is about 1.1k instructions per D3Q19 cell and 1.9k per D3Q27
+// cell, so the plain one-cell-per-thread kernel spends its time either issuing or
+// waiting on its 19/27 loads.  Here every warp is persistent and works on tiles of
+// 32 consecutive cells: while it collides tile k it already has the loads of tile
+// k+1 in flight as cp.async copies (8 bytes per thread and direction) into its own
+// two-stage shared-memory buffer, so the loads hold no registers and their latency
+// overlaps the collision.  Each thread reads back only what it copied itself, so
+// cp.async.wait_group is the only synchronisation needed.
 //
 // AA (in place) stays race-free under the prefetch: the locations a cell's
 // thread reads are exactly the ones it writes (even step: its own slots; odd
@@ -68,12 +67,15 @@ constexpr size_t async_smem_bytes()
    return (size_t)async_warps<Q, REST>() * kAsyncStages * async_rows<Q, REST>() * 32 * sizeof(unsigned long long);
 }
 
-// Tiles of 32 cells: tile t covers x in [32 (t mod ntx), +32) of row t / ntx,
-// row r = y + ny z, with ntx = ceil(nx / 32) (lanes past the row end idle).  Divisions by a run-time d use q = umulhi64(n, m) with
-// m = ceil(2^64 / d) (exact for n, d < 2^32); d = 1 is m = 0.
+// Tiles of 32 consecutive cells, whatever rows they lie in: tile t covers the cells
+// c in [32 t, 32 t + 32) below ncell.  Every lane has a cell then, and every tile
+// starts on 256 bytes; with tiles that ended at their rows, rows of 161 cells left
+// 16 % of the lanes idle (D3Q27 AB pull channel 161x75x93, two steps: 196 us).
+// Divisions by a run-time d use q = umulhi64(n, m) with m = ceil(2^64 / d) (exact for
+// n, d < 2^32); d = 1 is m = 0.
 struct AsyncGeom {
-   uint32_t ntiles, ntx;
-   uint64_t m_ntx, m_ny;
+   uint32_t ntiles, ncell;
+   uint64_t m_nx, m_ny;
 };
 
 __device__ __forceinline__ uint32_t div_magic(uint32_t n, uint32_t d, uint64_t m)
@@ -81,15 +83,16 @@ __device__ __forceinline__ uint32_t div_magic(uint32_t n, uint32_t d, uint64_t m
    return m ? (uint32_t)__umul64hi((uint64_t)n, m) : n;
 }
 
-// Returns false for a lane past the end of its row.
+// Returns false for a lane past the last cell.
 __device__ __forceinline__ bool tile_cell(const KParams& p, const AsyncGeom& ag, uint32_t t, int lane,
                                           CellIndex& ci)
 {
-   const uint32_t row = div_magic(t, ag.ntx, ag.m_ntx);
-   const int x = (int)(t - row * ag.ntx) * 32 + lane;
+   const uint32_t c = t * 32u + (uint32_t)lane;
+   const uint32_t row = div_magic(c, (uint32_t)p.nx, ag.m_nx);
+   const int x = (int)(c - row * (uint32_t)p.nx);
    const uint32_t z = div_magic(row, (uint32_t)p.ny, ag.m_ny);
    const int y = (int)(row - z * (uint32_t)p.ny);
-   ci.c = (int64_t)row * p.nx + x;
+   ci.c = (int64_t)c;
    ci.dxm = (x == 0) ? p.nx - 1 : -1;
    ci.dxp = (x == p.nx - 1) ? -(p.nx - 1) : 1;
    ci.dym = (y == 0) ? (p.ny - 1) * p.nx : -p.nx;
@@ -97,7 +100,7 @@ __device__ __forceinline__ bool tile_cell(const KParams& p, const AsyncGeom& ag,
    const int nxy = p.nx * p.ny;
    ci.dzm = (z == 0) ? (p.nz - 1) * nxy : -nxy;
    ci.dzp = ((int)z == p.nz - 1) ? -(p.nz - 1) * nxy : nxy;
-   return x < p.nx;
+   return c < ag.ncell;
 }
 
 __device__ __forceinline__ void cp_async8(uint32_t smem, const void* g)
@@ -118,25 +121,24 @@ struct PlanePtrs {
 };
 
 // Lane state of a tile: its cell, its link word (0 without walls) and
-// whether it updates anything (inside the row, not solid).
+// whether it updates anything (a cell, not solid).
 struct TileLane {
    CellIndex ci;
    uint32_t lk;
    bool active;
 };
 
-// Link word of this lane's cell in tile t (the solid bit past the row end).
+// Link word of this lane's cell in tile t (the solid bit past the last cell).
 __device__ __forceinline__ uint32_t tile_link(const KParams& p, const AsyncGeom& ag, uint32_t t, int lane)
 {
-   const uint32_t row = div_magic(t, ag.ntx, ag.m_ntx);
-   const int x = (int)(t - row * ag.ntx) * 32 + lane;
-   return x < p.nx ? __ldg(p.links + (int64_t)row * p.nx + x) : kSolidBit;
+   const uint32_t c = t * 32u + (uint32_t)lane;
+   return c < ag.ncell ? __ldg(p.links + c) : kSolidBit;
 }
 
 // lk: the tile's link words, loaded one tile ahead so the load's latency
 // hides behind a collision.
-// RAGGED: nx is not a multiple of 32, so some lanes fall past their row (with
-// LINKS their link word says so, and RAGGED is not looked at).
+// RAGGED: the cell count is not a multiple of 32, so the last tile has lanes
+// without a cell (with LINKS their link word says so, and RAGGED is not looked at).
 template <bool LINKS, bool RAGGED>
 __device__ __forceinline__ void tile_lane(const KParams& p, const AsyncGeom& ag, uint32_t t, int lane, uint32_t lk,
                                           TileLane& tl)
@@ -265,9 +267,9 @@ __global__ void __launch_bounds__(async_warps<Q, REST>() * 32, async_min_blocks<
 inline AsyncGeom async_geom(int nx, int ny, int nz)
 {
    AsyncGeom g;
-   g.ntx = (uint32_t)((nx + 31) / 32);
-   g.ntiles = g.ntx * (uint32_t)ny * (uint32_t)nz;
-   g.m_ntx = g.ntx == 1 ? 0 : (~0ull / g.ntx) + 1;
+   g.ncell = (uint32_t)nx * (uint32_t)ny * (uint32_t)nz;   // below 2^31
+   g.ntiles = g.ncell / 32u + (g.ncell % 32u ? 1u : 0u);
+   g.m_nx = nx == 1 ? 0 : (~0ull / (uint64_t)nx) + 1;
    g.m_ny = ny == 1 ? 0 : (~0ull / (uint64_t)ny) + 1;
    return g;
 }
@@ -352,13 +354,13 @@ cudaError_t launch_async_form(const KParams& p, const AsyncGeom& ag, const void*
 }
 
 // links: the grid has link words.  Kernels exist for no force and the velocity
-// shift with full and ragged rows; the other forcing forms run the ragged form
-// for every row length.
+// shift with and without a ragged last tile; the other forcing forms run the
+// ragged form for every cell count.
 template <int Q, int KIND>
 cudaError_t launch_async_kind(bool links, const KParams& p, const AsyncGeom& ag, const void* src, void* dst,
                               cudaStream_t stream)
 {
-   const bool ragged = p.nx % 32 != 0;
+   const bool ragged = ag.ncell % 32u != 0u;
    if (p.forced == 0) {
       if (links) return launch_async_form<Q, KIND, true, false, 0>(p, ag, src, dst, stream);
       return ragged ? launch_async_form<Q, KIND, false, true, 0>(p, ag, src, dst, stream)

@@ -1,9 +1,9 @@
 // Software-pipelined step kernel for the shifted FP32 / BF16 / FP16 storage
-// (FP32 collision), for any box: link words for walls and solids, rows of
-// any length, no per-cell fields.
+// (FP32 collision), for boxes with link words (walls and solids), rows of any
+// length, no per-cell fields.
 //
 // Same scheme as the FP64 pipelined kernel (lbm_step_async.cuh): persistent
-// warps on tiles of 32 consecutive cells of one x row, one cell per lane;
+// warps on tiles of 32 consecutive cells, one cell per lane;
 // while a warp collides tile k, the populations of tile k+1 are already in
 // flight as cp.async copies into the warp's two-stage shared-memory buffer.
 // cp.async moves 4, 8 or 16 bytes, so each lane copies the aligned 4-byte
@@ -59,17 +59,17 @@ __device__ __forceinline__ float word_value(uint32_t w, bool high)
 
 // Issue the copies of one lane's populations; returns the word-half mask
 // (bit s set: direction s sits in the high half of its word).
-template <int Q, int ST, int KIND, bool LINKS, bool RAGGED>
+template <int Q, int ST, int KIND>
 __device__ __forceinline__ uint32_t async_issue_low(const PlanePtrsT<typename Store<ST>::T>& pp, const TileLane& tl,
                                                     int lane, uint32_t sbuf)
 {
    using T = typename Store<ST>::T;
    uint32_t halves = 0u;
-   if ((LINKS || RAGGED) && !tl.active) return halves;
+   if (!tl.active) return halves;
    const uint32_t c = (uint32_t)tl.ci.c;
 #pragma unroll
    for (int s = 0; s < Q; s++) {
-      const Access a = read_access<Q, KIND, LINKS>(tl.ci, tl.lk, s);
+      const Access a = read_access<Q, KIND, true>(tl.ci, tl.lk, s);
       const uint32_t e = c + (uint32_t)a.off;
       const T* elem = pp.src + ((uint32_t)a.slot * pp.plane + e);
       const void* word = elem;
@@ -82,7 +82,7 @@ __device__ __forceinline__ uint32_t async_issue_low(const PlanePtrsT<typename St
    return halves;
 }
 
-template <int Q, int ST, int KIND, bool LINKS, bool RAGGED>
+template <int Q, int ST, int KIND>
 __global__ void __launch_bounds__(kAsyncLowWarps * 32) step_async_low_kernel(
    const KParams p, const AsyncGeom ag, const PlanePtrsT<typename Store<ST>::T> pp)
 {
@@ -104,23 +104,23 @@ __global__ void __launch_bounds__(kAsyncLowWarps * 32) step_async_low_kernel(
       uint32_t t1 = t + nw < ntiles ? t + nw : ntiles;
       uint32_t t2 = t + 2u * nw < ntiles ? t + 2u * nw : ntiles;
       TileLane cur;
-      tile_lane<LINKS, RAGGED>(p, ag, t, lane, LINKS ? tile_link(p, ag, t, lane) : 0u, cur);
-      uint32_t lk_ahead = (LINKS && t1 < ntiles) ? tile_link(p, ag, t1, lane) : 0u;
-      uint32_t halves = async_issue_low<Q, ST, KIND, LINKS, RAGGED>(pp, cur, lane, sbase);
+      tile_lane<true, false>(p, ag, t, lane, tile_link(p, ag, t, lane), cur);
+      uint32_t lk_ahead = t1 < ntiles ? tile_link(p, ag, t1, lane) : 0u;
+      uint32_t halves = async_issue_low<Q, ST, KIND>(pp, cur, lane, sbase);
       cp_async_commit();
       int stage = 0;
       for (;;) {
          TileLane nxt = cur;
          uint32_t halves_next = 0u;
          if (t1 < ntiles) {
-            tile_lane<LINKS, RAGGED>(p, ag, t1, lane, lk_ahead, nxt);
-            if (LINKS && t2 < ntiles) lk_ahead = tile_link(p, ag, t2, lane);
+            tile_lane<true, false>(p, ag, t1, lane, lk_ahead, nxt);
+            if (t2 < ntiles) lk_ahead = tile_link(p, ag, t2, lane);
             halves_next =
-               async_issue_low<Q, ST, KIND, LINKS, RAGGED>(pp, nxt, lane, sbase + (stage ^ 1) * kStageBytes);
+               async_issue_low<Q, ST, KIND>(pp, nxt, lane, sbase + (stage ^ 1) * kStageBytes);
          }
          cp_async_commit();
          cp_async_wait_prev();
-         if (!(LINKS || RAGGED) || cur.active) {
+         if (cur.active) {
             float g[Q], o[Q];
             const uint32_t* sm = mine + stage * Q * 32;
 #pragma unroll
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(kAsyncLowWarps * 32) step_async_low_kernel(
             const uint32_t c = (uint32_t)cur.ci.c;
 #pragma unroll
             for (int s = 0; s < Q; s++) {
-               const Access a = write_access<Q, KIND, LINKS>(cur.ci, cur.lk, s);
+               const Access a = write_access<Q, KIND, true>(cur.ci, cur.lk, s);
                store_raw(pp.dst + ((uint32_t)a.slot * pp.plane + c + (uint32_t)a.off), o[s]);
             }
          }
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(kAsyncLowWarps * 32) step_async_low_kernel(
    if (fed) feed_done(p.sched);
 }
 
-template <int Q, int ST, int KIND, bool LINKS, bool RAGGED>
+template <int Q, int ST, int KIND>
 cudaError_t launch_async_low(const KParams& p, const AsyncGeom& ag, const void* src, void* dst, cudaStream_t stream)
 {
    using T = typename Store<ST>::T;
@@ -157,7 +157,7 @@ cudaError_t launch_async_low(const KParams& p, const AsyncGeom& ag, const void* 
    cudaError_t e = cudaGetDevice(&dev);
    if (e != cudaSuccess) return e;
    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-   auto kern = step_async_low_kernel<Q, ST, KIND, LINKS, RAGGED>;
+   auto kern = step_async_low_kernel<Q, ST, KIND>;
    constexpr size_t smem = async_low_smem_bytes<Q>();
    int cached = grid_of_device[dev].load(std::memory_order_relaxed);
    if (cached == 0) {
