@@ -40,10 +40,9 @@ namespace lbm {
 //          165 KB): odd 324 us, pull 295 us, even 291 us, push 303 us (links 317);
 //   else   one block, all directions staged: odd 342, pull 309, even 281, push
 //          302 us (links 308).
-// The gathers run the first; the others the second, but the first for grids of
-// fewer than 16 tiles per warp, where a step overlaps the next by the block (48^3:
-// AA 11.5 us a step against 13.6, push 11.6 against 13.7).  D3Q19 with a rest
-// register: 201 / 219 us, so not there.
+// AA odd and AB run the first; AA even the second, but the first for grids of fewer
+// than 16 tiles per warp, where a step overlaps the next by the block (48^3: 11.5 us
+// a step against 13.6).  D3Q19 with a rest register: 201 / 219 us, so not there.
 template <int Q, bool REST>
 constexpr int async_warps() { return Q == 19 ? 8 : (REST ? 4 : 12); }
 template <int Q, bool REST>
@@ -51,6 +50,15 @@ constexpr int async_min_blocks() { return Q == 19 ? 2 : (REST ? 3 : 1); }
 // Directions staged in shared memory per tile.
 template <int Q, bool REST>
 constexpr int async_rows() { return REST ? Q - 1 : Q; }
+// Whether a block's warps take adjacent tiles at the same time, one barrier per
+// tile.  A D3Q27 AB step moves 54 streams; once its warps have drifted apart, each
+// 256-byte piece of a stream comes at a time of its own, and DRAM falls from 6.1
+// to 4.2 TB/s: the 256x128x128 pull channel took 291 or 423 us a step, from one run
+// to the next and within a run, and push 303 or 413 us.  Kept together in fours: 297
+// us whatever came before (box 292 -> 299).  AA reads and writes one set of 27
+// streams and does not fall; the barrier costs it 10 %.
+template <int Q, int KIND>
+constexpr bool async_together() { return Q == 27 && (KIND == K_AB_PUSH || KIND == K_AB_PULL); }
 constexpr int kAsyncStages = 2;
 constexpr int kBlockReserve = 1024;          // shared memory the system takes per block
 constexpr int kMaxSharedPerSM = 228 * 1024;
@@ -211,57 +219,135 @@ __global__ void __launch_bounds__(async_warps<Q, REST>() * 32, async_min_blocks<
    unsigned long long* mine = async_smem + (size_t)warp * kAsyncStages * kRows * 32;
    const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(mine);
    constexpr uint32_t kStageBytes = kRows * 32 * 8;
-   // tiles: three per warp in a fixed order, then the launch's tile feed (8
-   // counters for the D3Q19 tiles, which it hands out fastest); t is collided
-   // while t1's populations are in flight and t2's link words are loaded
-   const bool fed = feed_on(ntiles, nw);
-   TileFeed feed{0u, 0u, 1u, false};
-   if (fed) feed = feed_start(p.sched, 3u * nw, ntiles, blockIdx.x * kWarps + warp, nw, Q == 19 ? kFeedGroups : 1u, lane);
-   uint32_t t = blockIdx.x * kWarps + warp;
-   if (t < ntiles) {
-      uint32_t t1 = t + nw < ntiles ? t + nw : ntiles;
-      uint32_t t2 = t + 2u * nw < ntiles ? t + 2u * nw : ntiles;
-      TileLane cur;
-      tile_lane<LINKS, RAGGED>(p, ag, t, lane, LINKS ? tile_link(p, ag, t, lane) : 0u, cur);
-      uint32_t lk_ahead = (LINKS && t1 < ntiles) ? tile_link(p, ag, t1, lane) : 0u;
-      uint64_t rest = 0, rest_next = 0;
-      async_issue<Q, KIND, LINKS, RAGGED, REST>(pp, cur, lane, sbase, rest);
-      cp_async_commit();
-      int stage = 0;
-      for (;;) {
-         TileLane nxt = cur;
-         if (t1 < ntiles) {
-            tile_lane<LINKS, RAGGED>(p, ag, t1, lane, lk_ahead, nxt);
-            if (LINKS && t2 < ntiles) lk_ahead = tile_link(p, ag, t2, lane);
-            async_issue<Q, KIND, LINKS, RAGGED, REST>(pp, nxt, lane, sbase + (stage ^ 1) * kStageBytes, rest_next);
+   if constexpr (async_together<Q, KIND>()) {
+      // The block's warps take kWarps consecutive tiles together: group g is the
+      // tiles g kWarps + warp.  Three groups in a fixed order, then one counter,
+      // which the block's first thread asks one group ahead.  Everything about
+      // groups is block-uniform, a warp past the last tile only skips the work.
+      __shared__ uint32_t next_group[2];
+      const uint32_t nb = gridDim.x, ngroups = (ntiles + kWarps - 1) / kWarps;
+      const bool fed = feed_on(ntiles, nw);
+      uint32_t pend = 0;
+      if (fed && threadIdx.x == 0) pend = atomicAdd(p.sched, 1u);
+      uint32_t g = blockIdx.x, it = 0;
+      if (g < ngroups) {
+         uint32_t g1 = g + nb < ngroups ? g + nb : ngroups, g2 = g + 2u * nb < ngroups ? g + 2u * nb : ngroups;
+         auto tile = [&](uint32_t gg) { const uint32_t tt = gg * kWarps + warp; return gg < ngroups && tt < ntiles ? tt : ntiles; };
+         uint32_t t = tile(g), t1 = tile(g1), t2 = tile(g2);
+         TileLane cur;
+         cur.active = false;
+         cur.lk = kSolidBit;
+         uint64_t rest = 0, rest_next = 0;
+         if (t < ntiles) {
+            tile_lane<LINKS, RAGGED>(p, ag, t, lane, LINKS ? tile_link(p, ag, t, lane) : 0u, cur);
+            async_issue<Q, KIND, LINKS, RAGGED, REST>(pp, cur, lane, sbase, rest);
          }
+         uint32_t lk_ahead = (LINKS && t1 < ntiles) ? tile_link(p, ag, t1, lane) : 0u;
          cp_async_commit();
-         cp_async_wait_prev();
-         // each output is stored as the collision makes it, and the update
-         // re-reads its inputs from shared memory: neither the Q input nor the
-         // Q output patterns stay in registers
-         constexpr bool kScatters = KIND == K_AA_ODD || KIND == K_AB_PUSH;
-         const unsigned long long* in = mine + stage * kRows * 32 + lane;
-         const bool linked = LINKS && kScatters && tile_linked(cur.lk);
-         if (!(LINKS || RAGGED) || cur.active) {
-            if (LINKS && kScatters && linked) {
-               StoreEmit<Q, KIND, LINKS> emit{pp, cur.ci, cur.lk};
-               collide_f64x_shared_emit<Q, FORCE, REST>(in, rest, p, emit);
-            } else {
-               StoreEmit<Q, KIND, false> emit{pp, cur.ci, 0u};
-               collide_f64x_shared_emit<Q, FORCE, REST>(in, rest, p, emit);
+         int stage = 0;
+         for (;;) {
+            TileLane nxt = cur;
+            if (t1 < ntiles) {
+               tile_lane<LINKS, RAGGED>(p, ag, t1, lane, lk_ahead, nxt);
+               if (LINKS && t2 < ntiles) lk_ahead = tile_link(p, ag, t2, lane);
+               async_issue<Q, KIND, LINKS, RAGGED, REST>(pp, nxt, lane, sbase + (stage ^ 1) * kStageBytes, rest_next);
             }
+            cp_async_commit();
+            cp_async_wait_prev();
+            constexpr bool kScatters = KIND == K_AA_ODD || KIND == K_AB_PUSH;
+            const unsigned long long* in = mine + stage * kRows * 32 + lane;
+            if (t < ntiles) {
+               const bool linked = LINKS && kScatters && tile_linked(cur.lk);
+               if (!(LINKS || RAGGED) || cur.active) {
+                  if (LINKS && kScatters && linked) {
+                     StoreEmit<Q, KIND, LINKS> emit{pp, cur.ci, cur.lk};
+                     collide_f64x_shared_emit<Q, FORCE, REST>(in, rest, p, emit);
+                  } else {
+                     StoreEmit<Q, KIND, false> emit{pp, cur.ci, 0u};
+                     collide_f64x_shared_emit<Q, FORCE, REST>(in, rest, p, emit);
+                  }
+               }
+            }
+            if (g1 >= ngroups) break;
+            g = g1;
+            g1 = g2;
+            if (g2 < ngroups) {
+               if (fed) {
+                  if (threadIdx.x == 0) {
+                     const uint64_t n = 3ull * nb + pend;
+                     next_group[it & 1] = n < ngroups ? (uint32_t)n : ngroups;
+                     if (n < ngroups) pend = atomicAdd(p.sched, 1u);
+                  }
+                  __syncthreads();
+                  g2 = next_group[it & 1];
+               } else {
+                  g2 = g2 + nb < ngroups ? g2 + nb : ngroups;
+                  __syncthreads();
+               }
+            }
+            it++;
+            t = t1;
+            t1 = t2;
+            t2 = tile(g2);
+            cur = nxt;
+            rest = rest_next;
+            stage ^= 1;
          }
-         if (t1 >= ntiles) break;
-         t = t1;
-         t1 = t2;
-         t2 = feed_after(feed, fed, t2, p.sched, 3u * nw, ntiles, nw, lane);
-         cur = nxt;
-         rest = rest_next;
-         stage ^= 1;
       }
+      if (fed) feed_done(p.sched);
+   } else {
+      // tiles: three per warp in a fixed order, then the launch's tile feed (8
+      // counters for the D3Q19 tiles, which it hands out fastest); t is collided
+      // while t1's populations are in flight and t2's link words are loaded
+      const bool fed = feed_on(ntiles, nw);
+      TileFeed feed{0u, 0u, 1u, false};
+      if (fed) feed = feed_start(p.sched, 3u * nw, ntiles, blockIdx.x * kWarps + warp, nw, Q == 19 ? kFeedGroups : 1u, lane);
+      uint32_t t = blockIdx.x * kWarps + warp;
+      if (t < ntiles) {
+         uint32_t t1 = t + nw < ntiles ? t + nw : ntiles;
+         uint32_t t2 = t + 2u * nw < ntiles ? t + 2u * nw : ntiles;
+         TileLane cur;
+         tile_lane<LINKS, RAGGED>(p, ag, t, lane, LINKS ? tile_link(p, ag, t, lane) : 0u, cur);
+         uint32_t lk_ahead = (LINKS && t1 < ntiles) ? tile_link(p, ag, t1, lane) : 0u;
+         uint64_t rest = 0, rest_next = 0;
+         async_issue<Q, KIND, LINKS, RAGGED, REST>(pp, cur, lane, sbase, rest);
+         cp_async_commit();
+         int stage = 0;
+         for (;;) {
+            TileLane nxt = cur;
+            if (t1 < ntiles) {
+               tile_lane<LINKS, RAGGED>(p, ag, t1, lane, lk_ahead, nxt);
+               if (LINKS && t2 < ntiles) lk_ahead = tile_link(p, ag, t2, lane);
+               async_issue<Q, KIND, LINKS, RAGGED, REST>(pp, nxt, lane, sbase + (stage ^ 1) * kStageBytes, rest_next);
+            }
+            cp_async_commit();
+            cp_async_wait_prev();
+            // each output is stored as the collision makes it, and the update
+            // re-reads its inputs from shared memory: neither the Q input nor the
+            // Q output patterns stay in registers
+            constexpr bool kScatters = KIND == K_AA_ODD || KIND == K_AB_PUSH;
+            const unsigned long long* in = mine + stage * kRows * 32 + lane;
+            const bool linked = LINKS && kScatters && tile_linked(cur.lk);
+            if (!(LINKS || RAGGED) || cur.active) {
+               if (LINKS && kScatters && linked) {
+                  StoreEmit<Q, KIND, LINKS> emit{pp, cur.ci, cur.lk};
+                  collide_f64x_shared_emit<Q, FORCE, REST>(in, rest, p, emit);
+               } else {
+                  StoreEmit<Q, KIND, false> emit{pp, cur.ci, 0u};
+                  collide_f64x_shared_emit<Q, FORCE, REST>(in, rest, p, emit);
+               }
+            }
+            if (t1 >= ntiles) break;
+            t = t1;
+            t1 = t2;
+            t2 = feed_after(feed, fed, t2, p.sched, 3u * nw, ntiles, nw, lane);
+            cur = nxt;
+            rest = rest_next;
+            stage ^= 1;
+         }
+      }
+      if (fed) feed_done(p.sched);
    }
-   if (fed) feed_done(p.sched);
 }
 
 inline AsyncGeom async_geom(int nx, int ny, int nz)
@@ -337,8 +423,7 @@ template <int Q, int KIND, bool LINKS, bool RAGGED, int FORCE>
 cudaError_t launch_async_form(const KParams& p, const AsyncGeom& ag, const void* src, void* dst, cudaStream_t stream)
 {
    if constexpr (Q == 27) {
-      constexpr bool kGathers = KIND == K_AA_ODD || KIND == K_AB_PULL;
-      if constexpr (kGathers || FORCE == kForceOther) {
+      if constexpr (KIND != K_AA_EVEN || FORCE == kForceOther) {
          return launch_async_kernel<Q, KIND, LINKS, RAGGED, FORCE, true>(p, ag, src, dst, stream);
       } else {
          int dev = 0, nsm = 0;
@@ -349,7 +434,7 @@ cudaError_t launch_async_form(const KParams& p, const AsyncGeom& ag, const void*
             return launch_async_kernel<Q, KIND, LINKS, RAGGED, FORCE, true>(p, ag, src, dst, stream);
       }
    }
-   if constexpr (Q == 19 || !(KIND == K_AA_ODD || KIND == K_AB_PULL || FORCE == kForceOther))
+   if constexpr (Q == 19 || (KIND == K_AA_EVEN && FORCE != kForceOther))
       return launch_async_kernel<Q, KIND, LINKS, RAGGED, FORCE, false>(p, ag, src, dst, stream);
 }
 
