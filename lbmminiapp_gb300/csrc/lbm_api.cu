@@ -1,5 +1,6 @@
 // C ABI implementation (include/lbm_gb300.h): handle lifetime, geometry,
 // initialisation, the time loop and readouts.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -856,18 +857,34 @@ lbm_status lbm_step(lbm_handle* h, int nsteps)
    return LBM_OK;
 }
 
-// Device address of `n` doubles of page-locked host memory, null for any other
-// memory.
+// Device address of `n` doubles that lie in one allocation (or registration) of
+// page-locked host memory, null for any other memory.
 static double* mapped_host(double* p, int64_t n)
 {
-   cudaPointerAttributes a, b;
-   if (cudaPointerGetAttributes(&a, p) != cudaSuccess || cudaPointerGetAttributes(&b, p + (n - 1)) != cudaSuccess) {
+   cudaPointerAttributes a;
+   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
       cudaGetLastError();
       return nullptr;
    }
-   if (a.type != cudaMemoryTypeHost || b.type != cudaMemoryTypeHost || !a.devicePointer || !b.devicePointer) return nullptr;
-   double* d = static_cast<double*>(a.devicePointer);
-   return static_cast<double*>(b.devicePointer) == d + (n - 1) ? d : nullptr;
+   if (a.type != cudaMemoryTypeHost || !a.devicePointer) return nullptr;
+   // the allocation's extent, which the runtime does not tell
+   using Query = CUresult (*)(void*, CUpointer_attribute, CUdeviceptr);
+   void* fn = nullptr;
+   cudaDriverEntryPointQueryResult found;
+   if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &fn, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+       found != cudaDriverEntryPointSuccess || !fn) {
+      cudaGetLastError();
+      return nullptr;
+   }
+   const Query query = reinterpret_cast<Query>(fn);
+   CUdeviceptr start = 0;
+   size_t size = 0;
+   const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(a.devicePointer);
+   if (query(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at) != CUDA_SUCCESS ||
+       query(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at) != CUDA_SUCCESS)
+      return nullptr;
+   if (at < start || (uint64_t)(at - start) + sizeof(double) * (uint64_t)n > (uint64_t)size) return nullptr;
+   return static_cast<double*>(a.devicePointer);
 }
 
 lbm_status lbm_get_macros(lbm_handle* h, double* rho, double* u)

@@ -44,12 +44,13 @@ __device__ __forceinline__ bool finite_bits(double x) { return ((uint32_t)__doub
 
 // load(s): the deviation f_s - w_s of direction s as a float (shifted storage) or
 // the bit pattern of f_s (FP64 storage).  regular(): rho and j are finite and rho
-// is not zero.
+// is not zero.  Other cells (a diverged state) are summed in FP64.
 template <int Q, int ST, class Load>
 struct CellMoments {
    x64::df s[4];   // drho, j
+   const Load& load;
 
-   __device__ __forceinline__ explicit CellMoments(const Load& load)
+   __device__ __forceinline__ explicit CellMoments(const Load& l) : load(l)
    {
 #pragma unroll
       for (int k = 0; k < 4; k++) s[k] = {0.f, 0.f};
@@ -75,9 +76,24 @@ struct CellMoments {
    }
    __device__ __forceinline__ void get(double& rho, double (&j)[3]) const
    {
-      rho = 1.0 + (widen(s[0].h) + widen(s[0].l));
+      if (regular()) {
+         rho = 1.0 + (widen(s[0].h) + widen(s[0].l));
 #pragma unroll
-      for (int d = 0; d < 3; d++) j[d] = widen(s[1 + d].h) + widen(s[1 + d].l);
+         for (int d = 0; d < 3; d++) j[d] = widen(s[1 + d].h) + widen(s[1 + d].l);
+         return;
+      }
+      // TwoSum makes NaN of an infinite population
+      rho = j[0] = j[1] = j[2] = 0.0;
+#pragma unroll
+      for (int r = 0; r < Q; r++) {
+         const double f = (double)load(r) + lat_w(Q, r);
+         rho += f;
+#pragma unroll
+         for (int d = 0; d < 3; d++) {
+            if (lat_c(Q, r, d) > 0) j[d] += f;
+            if (lat_c(Q, r, d) < 0) j[d] -= f;
+         }
+      }
    }
 };
 
