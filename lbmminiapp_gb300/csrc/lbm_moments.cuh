@@ -5,8 +5,9 @@
 // an integer or FP32 add for one, so sums made there (49 adds per D3Q19 cell)
 // bound a kernel that only reads populations.  Here FP64 storage is summed
 // exactly as 64-bit integers (images floor(f * 2^62) of populations in
-// [2^-31, 1); a cell with another value is summed in FP64), and the shifted
-// formats in error-free FP32 additions (TwoSum) of the deviations f - w.
+// [2^-31, 1); a cell with another value, or with rho from 2, is summed in FP64),
+// and the shifted formats in error-free FP32 additions (TwoSum) of the
+// deviations f - w.
 #pragma once
 
 #include "lbm_f64x.cuh"
@@ -104,18 +105,18 @@ struct CellMoments<Q, ST_F64, Load> {
    const Load& load;
 
    // floor(f * 2^62) for f in [2^-31, 1)
-   __device__ __forceinline__ static uint64_t image(uint64_t b)
+   __host__ __device__ __forceinline__ static uint64_t image(uint64_t b)
    {
       const uint32_t lo = (uint32_t)b, hi = (uint32_t)(b >> 32);
       const uint32_t top = x64::funnel_l(lo, (hi & 0x000FFFFFu) | 0x00100000u, 10), low = lo << 10;
       const uint32_t k = 1023u - (hi >> 20);   // 1 to 31 in the range
       return ((uint64_t)x64::funnel_r(top, 0u, k) << 32) | x64::funnel_r(low, top, k);
    }
-   __device__ __forceinline__ explicit CellMoments(const Load& l) : load(l)
+   __host__ __device__ __forceinline__ explicit CellMoments(const Load& l) : load(l)
    {
       constexpr uint32_t kMin = (uint32_t)(1023 - 31) << 20, kMax = (uint32_t)1023 << 20;
       const uint64_t fr = load(lat_rest(Q));
-      uint32_t least = (uint32_t)(fr >> 32), most = least;
+      uint32_t least = (uint32_t)(fr >> 32), most = least, wrapped = 0u;
       r = image(fr);
       m[0] = m[1] = m[2] = 0;
 #pragma unroll
@@ -126,17 +127,18 @@ struct CellMoments<Q, ST_F64, Load> {
          most = x64::max3u(most, (uint32_t)(fs >> 32), (uint32_t)(fo >> 32));
          const uint64_t X = image(fs), Y = image(fo), D = X - Y;
          r += X + Y;
+         // rho < 2, looked at after every pair: the sum cannot wrap in between
+         wrapped |= (uint32_t)(r >> 32);
 #pragma unroll
          for (int d = 0; d < 3; d++) {
             if (lat_c(Q, s, d) > 0) m[d] += D;
             if (lat_c(Q, s, d) < 0) m[d] -= D;
          }
       }
-      // rho < 2: no wrap
-      exact = least >= kMin && most < kMax && (r >> 63) == 0;
+      exact = least >= kMin && most < kMax && !(wrapped & 0x80000000u);
    }
-   __device__ __forceinline__ bool regular() const { return exact; }
-   __device__ __forceinline__ void get(double& rho, double (&j)[3]) const
+   __host__ __device__ __forceinline__ bool regular() const { return exact; }
+   __host__ __device__ __forceinline__ void get(double& rho, double (&j)[3]) const
    {
       if (exact) {
          rho = fixed62_to_double((int64_t)r);
