@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -857,8 +858,29 @@ lbm_status lbm_step(lbm_handle* h, int nsteps)
    return LBM_OK;
 }
 
-// Device address of `n` doubles that lie in one allocation (or registration) of
-// page-locked host memory, null for any other memory.
+// The driver's attribute query: the runtime tells neither an allocation's extent nor
+// what the device may do with it.  Looked up until it is found, then kept.
+using PointerQuery = CUresult (*)(void*, CUpointer_attribute, CUdeviceptr);
+static PointerQuery pointer_query()
+{
+   static std::atomic<PointerQuery> found{nullptr};
+   PointerQuery q = found.load(std::memory_order_relaxed);
+   if (q) return q;
+   void* fn = nullptr;
+   cudaDriverEntryPointQueryResult result;
+   if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &fn, 12000, cudaEnableDefault, &result) != cudaSuccess ||
+       result != cudaDriverEntryPointSuccess || !fn) {
+      cudaGetLastError();
+      return nullptr;
+   }
+   q = reinterpret_cast<PointerQuery>(fn);
+   found.store(q, std::memory_order_relaxed);
+   return q;
+}
+
+// Device address of `n` doubles that a kernel can store to: in one allocation (or
+// registration) of page-locked host memory, on an 8-byte boundary, writable by the
+// device.  Null for any other memory, which is copied to.
 static double* mapped_host(double* p, int64_t n)
 {
    cudaPointerAttributes a;
@@ -867,22 +889,18 @@ static double* mapped_host(double* p, int64_t n)
       return nullptr;
    }
    if (a.type != cudaMemoryTypeHost || !a.devicePointer) return nullptr;
-   // the allocation's extent, which the runtime does not tell
-   using Query = CUresult (*)(void*, CUpointer_attribute, CUdeviceptr);
-   void* fn = nullptr;
-   cudaDriverEntryPointQueryResult found;
-   if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &fn, 12000, cudaEnableDefault, &found) != cudaSuccess ||
-       found != cudaDriverEntryPointSuccess || !fn) {
-      cudaGetLastError();
-      return nullptr;
-   }
-   const Query query = reinterpret_cast<Query>(fn);
+   const PointerQuery query = pointer_query();
+   if (!query) return nullptr;
    CUdeviceptr start = 0;
    size_t size = 0;
+   unsigned long long access = 0;
    const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(a.devicePointer);
+   if (at % sizeof(double) != 0) return nullptr;
    if (query(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at) != CUDA_SUCCESS ||
-       query(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at) != CUDA_SUCCESS)
+       query(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at) != CUDA_SUCCESS ||
+       query(&access, CU_POINTER_ATTRIBUTE_ACCESS_FLAGS, at) != CUDA_SUCCESS)
       return nullptr;
+   if (access != CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE) return nullptr;
    if (at < start || (uint64_t)(at - start) + sizeof(double) * (uint64_t)n > (uint64_t)size) return nullptr;
    return static_cast<double*>(a.devicePointer);
 }
