@@ -674,6 +674,10 @@ static lbm_status set_field(lbm_handle* h, const double* host, int ncomp, double
          for (int64_t c = 0; c < h->ncell; c++) tmp[(size_t)c] = (float)host[(size_t)k * h->ncell + c];
          LBM_CUDA(h, cudaMemcpy(*d32 + (size_t)k * h->plane, tmp.data(), sizeof(float) * (size_t)h->ncell,
                                 cudaMemcpyHostToDevice));
+         // the FP64 array that lbm_set_fields_device made for the loss and the adjoint
+         if (*d64)
+            LBM_CUDA(h, cudaMemcpyAsync(*d64 + (size_t)k * h->plane, host + (size_t)k * h->ncell,
+                                        sizeof(double) * (size_t)h->ncell, cudaMemcpyHostToDevice, h->stream));
       }
    }
    LBM_CUDA(h, cudaStreamSynchronize(h->stream));
