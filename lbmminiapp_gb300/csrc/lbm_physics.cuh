@@ -111,9 +111,10 @@ __host__ __device__ constexpr int pair_rep()
 // S enters only through per-cell factors.  Opposite directions share
 // cu(opp) = -cu, so S (eq - w) = A +- B with A = w (S drho + S rho (cu^2 - uu)/2)
 // and B = w S rho cu.
-// Every operation is written with its own rounding (products joined to sums by
-// explicit multiply-adds), so that the one-cell and the two-cell forms, in any
-// kernel, give the same bits.
+// Every operation has a rounding of its own, whatever the compiler contracts:
+// products are joined to sums by explicit multiply-adds, and sums of values that
+// are products themselves (3u, 3F) are intrinsics.  So the one-cell and the
+// two-cell forms, in any kernel, give the same bits.
 template <int ST> struct ShiftScale { static constexpr float S = 1.0f; };
 template <> struct ShiftScale<ST_F16> { static constexpr float S = kF16Scale; };
 
@@ -131,8 +132,8 @@ __device__ __forceinline__ float cdot_f(const float (&v)[3])
    float r = 0.0f;
    bool any = false;
    if (c0 != 0) { r = c0 > 0 ? v[0] : -v[0]; any = true; }
-   if (c1 != 0) { r = any ? (c1 > 0 ? r + v[1] : r - v[1]) : (c1 > 0 ? v[1] : -v[1]); any = true; }
-   if (c2 != 0) { r = any ? (c2 > 0 ? r + v[2] : r - v[2]) : (c2 > 0 ? v[2] : -v[2]); }
+   if (c1 != 0) { r = any ? (c1 > 0 ? x64::fadd(r, v[1]) : x64::fsub(r, v[1])) : (c1 > 0 ? v[1] : -v[1]); any = true; }
+   if (c2 != 0) { r = any ? (c2 > 0 ? x64::fadd(r, v[2]) : x64::fsub(r, v[2])) : (c2 > 0 ? v[2] : -v[2]); }
    return r;
 }
 
@@ -195,8 +196,8 @@ __device__ __forceinline__ void shifted_pair(const ShiftedCell& c, float Gs, flo
       constexpr float w = (float)lat_w(Q, s);
       const float cf = cdot_f<Q, s>(c.F3);
       const float sym = fmaf(cu, cf, -c.fu);
-      fs = Som2 * w * (cf + sym);
-      fo = Som2 * w * (sym - cf);
+      fs = Som2 * w * x64::fadd(cf, sym);
+      fo = Som2 * w * x64::fsub(sym, cf);
    }
    os = fmaf(om1, Gs, fmaf(omega, fmaf(c.wSr[cls], cu, A), fs));
    oob = fmaf(om1, Gob, fmaf(omega, fmaf(-c.wSr[cls], cu, A), fo));
@@ -239,7 +240,7 @@ __device__ __forceinline__ void collide_f32(const float (&G)[Q], float (&o)[Q], 
    if (sp != 0.0f) {
       const float keep = 1.0f - sp;
 #pragma unroll
-      for (int s = 0; s < Q; s++) o[s] = keep * o[s] + sp * G[lat_opp(Q, s)];
+      for (int s = 0; s < Q; s++) o[s] = fmaf(keep, o[s], x64::fmul(sp, G[lat_opp(Q, s)]));
    }
 }
 
