@@ -4,13 +4,13 @@
 // One FP64 instruction holds its pipe for 76 cycles per warp and sub-partition,
 // an integer or FP32 add for one, so sums made there (49 adds per D3Q19 cell)
 // bound a kernel that only reads populations.  Here FP64 storage is summed
-// exactly as 64-bit integers (images floor(f * 2^62) of populations in
-// [2^-31, 1); a cell with another value, or with rho from 2, is summed in FP64),
+// exactly as 64-bit integers (images f * 2^62 of populations in [2^-10, 1), which
+// lose no bit; a cell with another value, or with rho from 2, is summed in FP64),
 // and the shifted formats in error-free FP32 additions (TwoSum) of the
 // deviations f - w.
 #pragma once
 
-#include "lbm_f64x.cuh"
+#include "lbm_soft.cuh"
 
 namespace lbm {
 
@@ -104,20 +104,12 @@ struct CellMoments<Q, ST_F64, Load> {
    bool exact;
    const Load& load;
 
-   // floor(f * 2^62) for f in [2^-31, 1)
-   __host__ __device__ __forceinline__ static uint64_t image(uint64_t b)
-   {
-      const uint32_t lo = (uint32_t)b, hi = (uint32_t)(b >> 32);
-      const uint32_t top = x64::funnel_l(lo, (hi & 0x000FFFFFu) | 0x00100000u, 10), low = lo << 10;
-      const uint32_t k = 1023u - (hi >> 20);   // 1 to 31 in the range
-      return ((uint64_t)x64::funnel_r(top, 0u, k) << 32) | x64::funnel_r(low, top, k);
-   }
    __host__ __device__ __forceinline__ explicit CellMoments(const Load& l) : load(l)
    {
-      constexpr uint32_t kMin = (uint32_t)(1023 - 31) << 20, kMax = (uint32_t)1023 << 20;
+      constexpr uint32_t kMin = (uint32_t)(1023 - 10) << 20, kMax = (uint32_t)1023 << 20;
       const uint64_t fr = load(lat_rest(Q));
       uint32_t least = (uint32_t)(fr >> 32), most = least, wrapped = 0u;
-      r = image(fr);
+      r = soft::image(fr);
       m[0] = m[1] = m[2] = 0;
 #pragma unroll
       for (int q = 0; q < (Q - 1) / 2; q++) {
@@ -125,7 +117,7 @@ struct CellMoments<Q, ST_F64, Load> {
          const uint64_t fs = load(s), fo = load(o);
          least = x64::min3u(least, (uint32_t)(fs >> 32), (uint32_t)(fo >> 32));
          most = x64::max3u(most, (uint32_t)(fs >> 32), (uint32_t)(fo >> 32));
-         const uint64_t X = image(fs), Y = image(fo), D = X - Y;
+         const uint64_t X = soft::image(fs), Y = soft::image(fo), D = X - Y;
          r += X + Y;
          // rho < 2, looked at after every pair: the sum cannot wrap in between
          wrapped |= (uint32_t)(r >> 32);

@@ -82,3 +82,14 @@ def test_any_populations_below_one(lib, Q):
     out, regular = moments_f64(lib, Q, f)
     assert regular.any() and not regular.all()
     assert largest_error(Q, f, out) <= 1
+
+
+@pytest.mark.parametrize("Q", [19, 27])
+@pytest.mark.parametrize("scale", [1e-1, 1e-3, 1e-5, 1e-7])
+def test_thin_cells(lib, Q, scale):
+    """Populations down to 2^-31 and below, all of them small or one alone."""
+    rng = np.random.default_rng(Q)
+    f = equilibrium(Q, np.ones(200), (0.05, -0.02, 0.01)) * (1 + 1e-3 * rng.standard_normal((200, Q)))
+    f[:100] *= scale
+    f[np.arange(100, 200), rng.integers(0, Q, 100)] *= scale
+    assert largest_error(Q, f, moments_f64(lib, Q, f)[0]) <= 1
