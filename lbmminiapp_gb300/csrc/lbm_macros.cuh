@@ -12,7 +12,7 @@ namespace lbm {
 // for export_plane_kernel: 0 slot s holds direction s, 1 slot opp(s) does, 2 pull
 // gather.  FP64 storage: the sums are the reference's, rounded after every
 // addition, so that the readout of equal populations is equal text; the shifted
-// formats are summed error-free (CellMoments).
+// formats are summed in integers and rounded once (CellMoments).
 //
 // Bound by the host link for page-locked arrays (67 MB at 189 GB/s for 128^3).
 // With the 49 adds per cell on the FP64 pipe the kernel alone took 290 us there.

@@ -93,3 +93,96 @@ def test_thin_cells(lib, Q, scale):
     f[:100] *= scale
     f[np.arange(100, 200), rng.integers(0, Q, 100)] *= scale
     assert largest_error(Q, f, moments_f64(lib, Q, f)[0]) <= 1
+
+
+def moments_shifted(lib, Q, g, f16=False):
+    g = np.ascontiguousarray(g)
+    out, regular = np.empty((len(g), 4)), np.empty(len(g), np.uint8)
+    lib.moments_shifted(Q, int(f16), P(g.ctypes.data), len(g), P(out.ctypes.data), P(regular.ctypes.data))
+    return out, regular.astype(bool)
+
+
+def errors_shifted(Q, g, out):
+    """|out - exact| of rho = 1 + sum g and j = sum c g, [n][4]."""
+    rows = exact(Q, g.astype(np.float64))
+    return np.array([[abs(float(Fraction(a) - (b + (k == 0)))) for k, (a, b) in enumerate(zip(got.tolist(), want))]
+                     for got, want in zip(out, rows)])
+
+
+def sums_fp64(Q, g):
+    """rho and j of f = g + w, added up in FP64 one after another."""
+    c, _, w = core.stencil(Q)
+    out = np.zeros((len(g), 4))
+    for s in range(Q):
+        f = g[:, s].astype(np.float64) + w[s]
+        out[:, 0] += f
+        for d in range(3):
+            out[:, 1 + d] += c[s][d] * f
+    return out
+
+
+def as_stored(g, f16):
+    """Deviations as the storage holds them (FP16: scaled by 2^15)."""
+    return (np.float16(g * 32768) / np.float32(32768)).astype(np.float32) if f16 else g
+
+
+def assert_as_accurate_as_fp64(lib, Q, g, f16=False):
+    """The largest and the mean error over the cells, of rho and of j, are no larger
+    than those of sums in FP64."""
+    out, regular = moments_shifted(lib, Q, g, f16)
+    e, ref = errors_shifted(Q, g, out), errors_shifted(Q, g, sums_fp64(Q, g))
+    if f16:
+        assert (regular == (g.sum(axis=1) > -0.5)).all()   # any state above density 1/2
+    for k in (slice(0, 1), slice(1, 4)):
+        assert e[:, k].max() <= ref[:, k].max()
+        assert e[:, k].mean() <= ref[:, k].mean()
+    return regular
+
+
+# spread of the deviations, density, velocity
+@pytest.mark.parametrize("Q", [19, 27])
+@pytest.mark.parametrize("noise,rho,U", [(1e-3, 1.0, 0.05), (1e-6, 1.0, 1e-4), (1e-2, 1.1, 0.15), (1e-2, 0.8, 0.1),
+                                         (3e-2, 1.25, 0.2), (1e-2, 2.5, 0.1), (1e-2, 5.0, 0.1)])
+@pytest.mark.parametrize("f16", [False, True])
+def test_shifted_sums_of_flow_cells(lib, Q, noise, rho, U, f16):
+    rng = np.random.default_rng(Q)
+    n = 300
+    u = rng.uniform(-U, U, (3, n))
+    f = core.equilibrium(Q, rho * (1 + 0.01 * rng.standard_normal(n)), u).T
+    g = as_stored((f - core.stencil(Q)[2] + f * noise * rng.standard_normal(f.shape)).astype(np.float32), f16)
+    regular = assert_as_accurate_as_fp64(lib, Q, g, f16)
+    if abs(rho - 1) <= 0.2:
+        assert regular.all()
+
+
+# exponents of the smallest and the largest deviation of a cell
+@pytest.mark.parametrize("Q", [19, 27])
+@pytest.mark.parametrize("least,most", [(-10, -6), (-20, -4), (-30, -4), (-45, -4), (-30, 0), (-20, 6), (-6, 20)])
+@pytest.mark.parametrize("f16", [False, True])
+def test_shifted_sums_of_spread_deviations(lib, Q, least, most, f16):
+    if f16 and most > 0:
+        pytest.skip("FP16 storage holds deviations below 2")
+    rng = np.random.default_rng(Q)
+    g = (np.exp2(rng.uniform(least, most, (300, Q))) * rng.choice([-1.0, 1.0], (300, Q))).astype(np.float32)
+    assert_as_accurate_as_fp64(lib, Q, as_stored(np.abs(g) if most >= 0 else g, f16), f16)
+
+
+@pytest.mark.parametrize("Q", [19, 27])
+def test_shifted_sums_at_the_edges(lib, Q):
+    """Zeros, subnormals, the smallest and largest deviations the integers take,
+    and the values that they leave to FP64."""
+    edges = np.float32([0.0, 1e-45, 2.0 ** -126, 2.0 ** -62, 2.0 ** -61, 2.0 ** -60, 2.0 ** -38, 2.0 ** -30, 0.01,
+                        np.nextafter(np.float32(0.125), np.float32(0)), 0.125, 0.3, 1e30, 3e38])
+    rows = [np.where(np.arange(Q) == k, sign * e, np.float32(0)) for e in edges for sign in (1, -1) for k in (0, 5, Q - 1)]
+    rows += [np.full(Q, sign * e) for e in edges[:-2] for sign in (1, -1)]
+    g = np.float32(rows)
+    out, regular = moments_shifted(lib, Q, g)
+    assert regular[np.abs(g).max(axis=1) < 0.02].all() and not regular[np.abs(g).max(axis=1) >= 0.125].any()
+    # per population: what a rounding of g + w in FP64 loses (half an ulp of 1/2 at most), and the sum's own rounding
+    tol = 2 * Q * 2.0 ** -53 * (1 + np.abs(g.astype(np.float64)).sum(axis=1))
+    assert (errors_shifted(Q, g, out).max(axis=1) <= tol).all()
+    for bad in (np.inf, -np.inf, np.nan):
+        g = np.zeros((1, Q), np.float32)
+        g[0, 3] = bad
+        out, regular = moments_shifted(lib, Q, g)
+        assert not regular[0] and not np.isfinite(out[0, 0])
