@@ -441,10 +441,14 @@ inline int force_mode(const double force[3], double omega)
 //   E_s = 3/2 F.F - (3 c.F)^2 / 2,
 // exactly: the forcing costs one multiply-add per pair instead of about 25
 // double-float operations.  The E term is single precision: with
-// sum |F_d| (1 - omega/2) / omega <= 1e-5 it is below 2^-28 of the equilibrium
-// (rho >= 1/4), its rounding below 2^-51.  Every workload of the benchmark lies
-// there.  Not for the rest weight of the Unroll kernels (compat), which breaks
-// the identity.
+// sum |F_d| (1 - omega/2) / omega <= 1e-5 and rho >= 1/4 it is below 2^-27 of the
+// equilibrium (|E| <= 4 (sum |F_d|)^2, at a diagonal force), and its error, from the
+// roundings of kappa, 1/rho, their product, its square and E, below 2^-48.  That is
+// at the limit and rho = 1/4; at rho = 1 both are 16 times smaller.  The whole
+// collision's error is below that of form 2, whose forcing terms are float pairs, at
+// any force up to the limit: rms over flow cells 8.2e-15 against 9.0e-15 (D3Q19,
+// tau = 0.55), 9.6e-15 against 1.07e-14 (D3Q27).  Not for the rest weight of the
+// Unroll kernels (compat), which breaks the identity.
 inline bool force_shifts(const double force[3], double omega)
 {
    double fsum = 0.0;
