@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include "lbm_aux.cuh"
+#include "lbm_step_async.cuh"
 
 namespace lbm {
 
@@ -35,7 +36,8 @@ struct AdjParams {
    int collide;                   // 0: loss term only (the last state of a rollout)
    const float* lam_next_f;       // FP32 adjoint: [Q][plane]
    float* lam_f;                  // FP32 adjoint: [Q][plane]
-   AdjConsts<double> k;           // set by the launch functions
+   AsyncGeom ag;                  // this and the constants: set by the launch functions
+   AdjConsts<double> k;
    AdjConsts<float> kf;
 };
 
