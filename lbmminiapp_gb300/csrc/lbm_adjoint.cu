@@ -37,9 +37,12 @@
 // and opposite directions enter them by their sum and difference.  That is about
 // 265 operations per D3Q19 cell; direction by direction it was 1180, and the
 // FP64 form is bound by the FP64 pipe (76 cycles per instruction, warp and
-// sub-partition).  Everything is written on the deviations g_s = f_s - w_s (the
-// shifted storage formats hold exactly these), so that f_opp(s) - C_s has no
-// cancellation against w.
+// sub-partition).  The sums over f run on deviations g_s = f_s - w_s r,
+//   sum_s mu_s (f_s - eq_s) = sum_s mu_s g_s - sum_s mu_s (eq_s - w_s r),
+// so that f_opp(s) - C_s has no cancellation against w r: r = 1 for the shifted
+// storage formats, which hold exactly these, and in FP32; in FP64 on FP64 storage
+// r is the density that the rest population stands for, so that a cell of small
+// density loses no bits against 1.
 //
 // One kernel for both adjoints: R = double, and R = float with lam and the
 // arithmetic in FP32.  The gradients are accumulated in FP64 either way; f^t may
@@ -54,11 +57,17 @@
 
 namespace lbm {
 
-// Deviation g = f - w of a stored population.
+// Whether r is the cell's own, not 1.
 template <int ST, typename R>
-__device__ __forceinline__ R load_dev(const void* buf, int64_t idx, double w)
+constexpr bool adj_scaled() { return ST == ST_F64 && sizeof(R) == 8; }
+
+// A stored population (adj_scaled), or its deviation f - w.
+template <int ST, typename R>
+__device__ __forceinline__ R load_adj(const void* buf, int64_t idx, double w)
 {
-   if constexpr (ST == ST_F64) {
+   if constexpr (adj_scaled<ST, R>()) {
+      return static_cast<const double*>(buf)[idx];
+   } else if constexpr (ST == ST_F64) {
       return (R)(static_cast<const double*>(buf)[idx] - w);
    } else {
       return (R)load_shifted(static_cast<const typename Store<ST>::T*>(buf) + idx);
@@ -136,10 +145,17 @@ __global__ void __launch_bounds__(kAdjThreads) adjoint_step_kernel(const AdjPara
    }
    if (a.collide) mur = next[(int64_t)RD * plane + c];
 
-   // drho, j and the products with mu of the porosity gradient, in one pass over f:
-   // dot1 = sum over pairs (f_s - f_o)(mu_s - mu_o), dot0 = sum of (g_s + g_o)(mu_s + mu_o)
-   const R gr = load_dev<ST, R>(a.state, (int64_t)RD * plane + c, lat_w(Q, RD));
-   R drho = gr, j[3] = {R(0), R(0), R(0)}, dot1 = R(0), dot0 = R(0);
+   // sum g, j and the products with mu of the porosity gradient, in one pass: dot1 =
+   // sum over pairs (f_s - f_o)(mu_s - mu_o), dot0 = sum of (g_s + g_o)(mu_s + mu_o)
+   constexpr bool kScaled = adj_scaled<ST, R>();
+   R gr = load_adj<ST, R>(a.state, (int64_t)RD * plane + c, lat_w(Q, RD)), r = R(1);
+   if constexpr (kScaled) {
+      r = gr * (1.0 / lat_w(Q, RD));
+      gr -= lat_w(Q, RD) * r;
+   }
+   // g_s + g_o from the loaded pair
+   const auto pair_sum = [&](R vs, R vo, double w) { return kScaled ? (vs + vo) - R(2.0 * w) * r : vs + vo; };
+   R total = gr, j[3] = {R(0), R(0), R(0)}, dot1 = R(0), dot0 = R(0);
    R m0 = (R)lat_w(Q, RD) * mur, m1[3] = {R(0), R(0), R(0)}, md[3] = {R(0), R(0), R(0)}, mo_[3] = {R(0), R(0), R(0)};
    // axes
    {
@@ -148,19 +164,10 @@ __global__ void __launch_bounds__(kAdjThreads) adjoint_step_kernel(const AdjPara
       for (int k = 0; k < 3; k++) {
          const int s = 2 * k, o = 2 * k + 1;
          const double w = lat_w(Q, s);
-         R S, D;
-         if constexpr (ST == ST_F64 && sizeof(R) == 8) {
-            const double fs = static_cast<const double*>(a.state)[(int64_t)s * plane + c];
-            const double fo = static_cast<const double*>(a.state)[(int64_t)o * plane + c];
-            S = (fs + fo) - 2.0 * w;
-            D = fs - fo;
-         } else {
-            const R gs = load_dev<ST, R>(a.state, (int64_t)s * plane + c, w);
-            const R go = load_dev<ST, R>(a.state, (int64_t)o * plane + c, w);
-            S = gs + go;
-            D = gs - go;
-         }
-         drho += S;
+         const R gs = load_adj<ST, R>(a.state, (int64_t)s * plane + c, w);
+         const R go = load_adj<ST, R>(a.state, (int64_t)o * plane + c, w);
+         const R S = pair_sum(gs, go, w), D = gs - go;
+         total += S;
          j[k] = D;
          dot1 += D * d[k];
          dot0 += S * p[k];
@@ -182,18 +189,11 @@ __global__ void __launch_bounds__(kAdjThreads) adjoint_step_kernel(const AdjPara
 #pragma unroll
          for (int h = 0; h < 2; h++) {
             const int s = pair_dir(Q, q1 + h), o = lat_opp(Q, s);
-            if constexpr (ST == ST_F64 && sizeof(R) == 8) {
-               const double fs = static_cast<const double*>(a.state)[(int64_t)s * plane + c];
-               const double fo = static_cast<const double*>(a.state)[(int64_t)o * plane + c];
-               S[h] = (fs + fo) - 2.0 * w;
-               D[h] = fs - fo;
-            } else {
-               const R gs = load_dev<ST, R>(a.state, (int64_t)s * plane + c, w);
-               const R go = load_dev<ST, R>(a.state, (int64_t)o * plane + c, w);
-               S[h] = gs + go;
-               D[h] = gs - go;
-            }
-            drho += S[h];
+            const R gs = load_adj<ST, R>(a.state, (int64_t)s * plane + c, w);
+            const R go = load_adj<ST, R>(a.state, (int64_t)o * plane + c, w);
+            S[h] = pair_sum(gs, go, w);
+            D[h] = gs - go;
+            total += S[h];
             dot1 += D[h] * d[q1 + h];
             dot0 += S[h] * p[q1 + h];
          }
@@ -215,11 +215,11 @@ __global__ void __launch_bounds__(kAdjThreads) adjoint_step_kernel(const AdjPara
 #pragma unroll
       for (int h = 0; h < 4; h++) {
          const int q = 9 + h, s = pair_dir(Q, q), o = lat_opp(Q, s);
-         const R gs = load_dev<ST, R>(a.state, (int64_t)s * plane + c, w);
-         const R go = load_dev<ST, R>(a.state, (int64_t)o * plane + c, w);
-         const R S = gs + go, D = gs - go;
+         const R gs = load_adj<ST, R>(a.state, (int64_t)s * plane + c, w);
+         const R go = load_adj<ST, R>(a.state, (int64_t)o * plane + c, w);
+         const R S = pair_sum(gs, go, w), D = gs - go;
          const R cy = (R)lat_c(Q, s, 1), cz = (R)lat_c(Q, s, 2);   // +-1
-         drho += S;
+         total += S;
          j[0] += D;
          j[1] += cy * D;
          j[2] += cz * D;
@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(kAdjThreads) adjoint_step_kernel(const AdjPara
    R sig = R(0);
    if (sizeof(R) == 4 && a.porosity_f) sig = a.porosity_f[c];
    else if (a.porosity) sig = (R)a.porosity[c];
-   const R rho = R(1) + drho;
+   const R rho = r + total;
    const R ir = R(1) / rho;
    R u[3];
 #pragma unroll
@@ -283,9 +283,9 @@ __global__ void __launch_bounds__(kAdjThreads) adjoint_step_kernel(const AdjPara
          jm += m1[k] * j[k];
          Fm += m1[k] * F[k];
       }
-      // sum_s mu_s (f_opp(s) - C_s) = -dot1 + omega (sum mu g - sum mu (eq - w)) - om2 sum mu fd
+      // sum_s mu_s (f_opp(s) - C_s) = -dot1 + omega (sum mu g - sum mu (eq - w r)) - om2 sum mu fd
       const R mug = R(0.5) * (dot0 + dot1) + mur * gr;
-      const R mueq = (drho - R(1.5) * uu * rho) * m0 + R(3) * jm + R(4.5) * rho * uMu;
+      const R mueq = (total - R(1.5) * uu * rho) * m0 + R(3) * jm + R(4.5) * rho * uMu;
       const R mufd = R(3) * Fm - ffe;
       gsig = om * (mug - mueq) - dot1 - om2 * mufd;
    }
