@@ -33,11 +33,17 @@ cudaError_t launch_kind(const Launch& L, const KParams& p, const void* src, void
    T* d = static_cast<T*>(dst);
    if constexpr (ST != ST_F64) {
       if (L.pair && !links && !fields) {
-         if (L.idx32)
-            return launch_overlapped(step_pair_kernel<Q, ST, KIND, uint32_t>, L.pair_grid, L.pair_block, 0, L.stream,
-                                     p, s, d);
-         return launch_overlapped(step_pair_kernel<Q, ST, KIND, int64_t>, L.pair_grid, L.pair_block, 0, L.stream, p,
-                                  s, d);
+         auto launch = [&](auto kern) {
+            return launch_overlapped(kern, L.pair_grid, L.pair_block, 0, L.stream, p, s, d);
+         };
+         if constexpr (pair_packed<Q, ST, KIND>(false)) {
+            if (pair_packed<Q, ST, KIND>(p.forced != 0))
+               return L.idx32 ? launch(step_pair_kernel<Q, ST, KIND, true, uint32_t>)
+                              : launch(step_pair_kernel<Q, ST, KIND, true, int64_t>);
+         }
+         if constexpr (!pair_packed<Q, ST, KIND>(true))
+            return L.idx32 ? launch(step_pair_kernel<Q, ST, KIND, false, uint32_t>)
+                           : launch(step_pair_kernel<Q, ST, KIND, false, int64_t>);
       }
       if (L.async_low && links && !fields) {
          return launch_async_low<Q, ST, KIND>(p, L.ag, src, dst, L.stream);

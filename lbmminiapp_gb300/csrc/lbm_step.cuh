@@ -245,10 +245,19 @@ constexpr int pair_min_blocks() { return Q == 27 ? 2 : (Store<ST>::bytes == 2 ? 
 // 312 / 372 / 346 / 330 us for D3Q27, from 199 / - / 226 / 214 to 195 / - / 206 /
 // 215 us for D3Q19.  The D3Q19 AA odd step, which has neighbour addresses for its
 // reads and its writes, spills with it (244 -> 273 us), so its cells stay apart.
-template <int Q, int KIND>
-constexpr bool pair_packed() { return !(Q == 19 && KIND == K_AA_ODD); }
+// Nor does it fit the 64 registers of the D3Q19 16-bit steps once the forcing joins:
+// 256x256x128 FP16 push with a force 136 us packed, 122 us apart, pull 115 and 113 us
+// (without a force push takes 103 us packed, 113 us apart).  So there are both
+// kernels for those, each with the code for both launches: compiled for the one
+// alone, the packed push step without a force takes 107 us.
+template <int Q, int ST, int KIND>
+constexpr bool pair_packed(bool forced)
+{
+   return !(Q == 19 && (KIND == K_AA_ODD || (forced && Store<ST>::bytes == 2)));
+}
 
-template <int Q, int ST, int KIND, typename IT>
+// PACKED for a launch with a force or without one as pair_packed() says.
+template <int Q, int ST, int KIND, bool PACKED, typename IT>
 __global__ void __launch_bounds__(256, pair_min_blocks<Q, ST>()) step_pair_kernel(const KParams p, const typename Store<ST>::T* src,
                                                         typename Store<ST>::T* dst)
 {
@@ -288,7 +297,7 @@ __global__ void __launch_bounds__(256, pair_min_blocks<Q, ST>()) step_pair_kerne
          *reinterpret_cast<typename PV::V*>(slot_ptr(d0, pb, a0)) = PV::put(o.x, o.y);
       }
    };
-   if constexpr (pair_packed<Q, KIND>()) {
+   if constexpr (PACKED) {
       if (p.forced) collide2_f32_emit<Q, ST, true>(g, p, emit);
       else collide2_f32_emit<Q, ST, false>(g, p, emit);
    } else {
