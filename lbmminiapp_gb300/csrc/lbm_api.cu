@@ -930,11 +930,11 @@ lbm_status lbm_get_macros(lbm_handle* h, double* rho, double* u)
    }
    st = ensure_copy_stream(h);
    if (st != LBM_OK) return st;
-   const int64_t chunk = chunk_cells(h, 4);
+   const int64_t chunk = chunk_cells(h, 4), nchunks = (n + chunk - 1) / chunk;
    const size_t half = h->staging_elems / 2;
    const void* buf = readout_buffer(h);
-   for (int64_t c0 = 0, k = 0; c0 < n; c0 += chunk, k++) {
-      const int64_t cnt = std::min<int64_t>(chunk, n - c0);
+   const auto compute = [&](int64_t k) -> lbm_status {
+      const int64_t c0 = k * chunk, cnt = std::min<int64_t>(chunk, n - c0);
       const int b = (int)(k & 1);
       double* part = h->staging + b * half;
       // the half is reused once its previous chunk has reached the host
@@ -942,6 +942,20 @@ lbm_status lbm_get_macros(lbm_handle* h, double* rho, double* u)
       dispatch_q_st<Macros>(h->Q, h->storage, h, c0, cnt, buf, mode, part, part + cnt, cnt);
       LBM_CUDA(h, cudaGetLastError());
       LBM_CUDA(h, cudaEventRecord(h->chunk_ready[b], h->stream));
+      return LBM_OK;
+   };
+   st = compute(0);
+   if (st != LBM_OK) return st;
+   for (int64_t k = 0; k < nchunks; k++) {
+      // the next chunk's kernel goes out first: a copy to pageable memory holds the
+      // host until it is done
+      if (k + 1 < nchunks) {
+         st = compute(k + 1);
+         if (st != LBM_OK) return st;
+      }
+      const int64_t c0 = k * chunk, cnt = std::min<int64_t>(chunk, n - c0);
+      const int b = (int)(k & 1);
+      double* part = h->staging + b * half;
       LBM_CUDA(h, cudaStreamWaitEvent(h->copy_stream, h->chunk_ready[b], 0));
       LBM_CUDA(h, cudaMemcpyAsync(rho + c0, part, sizeof(double) * cnt, cudaMemcpyDeviceToHost, h->copy_stream));
       for (int d = 0; d < 3; d++)
