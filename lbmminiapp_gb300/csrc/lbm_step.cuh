@@ -136,10 +136,16 @@ __device__ __forceinline__ void cell_force_f32(const KParams& p, int64_t c, floa
    }
 }
 
-// One launch = one time step (or one range of it) of one propagation kind.  The
-// exact FP64 arithmetic needs 16 warps per SM to keep its two pipes busy.
+// Blocks per SM that the registers have to leave room for: the exact FP64 arithmetic
+// needs 16 warps per SM to keep its two pipes busy, and F64X, whose kernels compile to
+// 128 registers or a little more, 16 to hide its loads.  Left to the compiler most of
+// those ran one block (range calls on 160x128x128: D3Q19 even step 186 us, 154 with
+// two; D3Q27 push with walls 467 us, 221 with two).
+constexpr int step_min_blocks(int arith) { return arith == AR_F32 ? 0 : 2; }
+
+// One launch = one time step (or one range of it) of one propagation kind.
 template <int Q, int ST, int AR, int KIND, bool LINKS, bool FIELDS, typename IT>
-__global__ void __launch_bounds__(256, AR == AR_F64 ? 2 : 0) step_kernel(const KParams p, const typename Store<ST>::T* src,
+__global__ void __launch_bounds__(256, step_min_blocks(AR)) step_kernel(const KParams p, const typename Store<ST>::T* src,
                                                    typename Store<ST>::T* dst)
 {
    wait_prior_grid();

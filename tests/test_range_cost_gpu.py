@@ -1,0 +1,48 @@
+"""F64X steps made by range calls against full steps, in time: the one-cell kernel of
+the ranges stays within 1.45 of the pipelined kernel (measured 1.15 to 1.3 with two
+blocks per SM, from 1.5 to 2.4 with one)."""
+import pytest
+
+from lbmminiapp_gb300 import Simulation
+
+pytestmark = pytest.mark.gpu
+
+
+def timed(call):
+    import torch
+    for _ in range(3):
+        call()
+    times = []
+    for _ in range(6):
+        first, last = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        torch.cuda.synchronize()
+        first.record()
+        for _ in range(8):
+            call()
+        last.record()
+        last.synchronize()
+        times.append(first.elapsed_time(last))
+    return min(times)
+
+
+@pytest.mark.parametrize("Q", [19, 27])
+@pytest.mark.parametrize("kind", ["even", "odd", "push", "pull"])
+@pytest.mark.parametrize("force", [0.0, 1e-6])
+def test_ranges_cost_little_more_than_steps(gpu, Q, kind, force):
+    import torch
+    pattern = "aa" if kind in ("even", "odd") else "ab_" + kind
+    with Simulation(160, 128, 128, lattice=Q, pattern=pattern, omega=1.4, force=(force, 0.0, 0.0)) as sim:
+        n, a = sim.ncell, sim.population_buffer()
+        other = torch.empty(int(sim.info.buffer_bytes), dtype=torch.uint8, device="cuda")
+
+        def run(parts):
+            for first, count in parts:
+                if kind == "even":
+                    sim.timestep_even_force(a, first, count)
+                elif kind == "odd":
+                    sim.timestep_odd_force(a, first, count)
+                else:
+                    sim.timestep_force(a, other.data_ptr(), first, count)
+
+        full = timed(lambda: run([(0, n)]))
+        assert timed(lambda: run([(0, n // 2), (n // 2, n - n // 2)])) <= 1.45 * full
