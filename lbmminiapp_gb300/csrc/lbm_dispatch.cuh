@@ -5,8 +5,6 @@
 
 #include <cuda_runtime.h>
 
-#include <type_traits>
-
 #include "lbm_step.cuh"
 #include "lbm_step_async.cuh"
 #include "lbm_step_async_low.cuh"
@@ -72,13 +70,14 @@ cudaError_t launch_kind(const Launch& L, const KParams& p, const void* src, void
    }
    // The exact FP64 arithmetic is bound by its pipe, not by addresses: 64-bit
    // strides only.
-   if (AR != AR_F64 && L.idx32) {
-      using IT = std::conditional_t<AR == AR_F64, int64_t, uint32_t>;
-      if (links)
-         return launch_overlapped(step_kernel<Q, ST, AR, KIND, true, false, IT>, L.grid, L.block, 0, L.stream, p,
+   if constexpr (AR != AR_F64) {
+      if (L.idx32) {
+         if (links)
+            return launch_overlapped(step_kernel<Q, ST, AR, KIND, true, false, uint32_t>, L.grid, L.block, 0, L.stream,
+                                     p, s, d);
+         return launch_overlapped(step_kernel<Q, ST, AR, KIND, false, false, uint32_t>, L.grid, L.block, 0, L.stream, p,
                                   s, d);
-      return launch_overlapped(step_kernel<Q, ST, AR, KIND, false, false, IT>, L.grid, L.block, 0, L.stream, p,
-                               s, d);
+      }
    }
    if (links)
       return launch_overlapped(step_kernel<Q, ST, AR, KIND, true, false, int64_t>, L.grid, L.block, 0, L.stream, p, s,

@@ -22,13 +22,14 @@ namespace lbm {
 //     the host;
 //   * without a force every forcing term is +-0 and leaves the result unchanged,
 //     unless v is not finite, which makes every result NaN (F.v = 0 inf).
-// Per D3Q19 cell: about 215 FP64 instructions without a force and 330 with one
-// (480 before).  The step kernels (SOFT) then move additions to the integer
-// pipes, which are idle: the sums, 1 + cu + cu^2/2 - uu/2 and the last addition
-// (lbm_soft.cuh), for cells in the ranges checked there; others take the plain
-// form.  About 94 FP64 instructions without a force: two steps of a 128^3 D3Q19
-// box took 3375 us with all 480, 1803 us with 215, 1183 us with 94 (the integer
-// work of about 3,500 instructions is the larger part then).
+// The step kernels (SOFT) then move additions to the integer pipes, which are idle:
+// the sums, 1 + cu + cu^2/2 - uu/2 and the last addition (lbm_soft.cuh), for cells in
+// the ranges checked there; others take the plain form.  Additions and products left
+// in FP64 per D3Q19 cell: 215 without a force and 330 with one in the plain form, 94
+// without a force in the integer one (136 executed with the reciprocal, by the
+// counter; the pipe is 78 % busy).  Two steps of a 128^3 D3Q19 box: 3375 us with
+// every operation of the reference, 1803 us in the plain form, 1182 us in the integer
+// one, whose integer work is about 3,500 instructions.
 template <int Q, int S>
 __device__ __forceinline__ double cdot_exact(double a0, double a1, double a2)
 {

@@ -153,23 +153,7 @@ __host__ __device__ __forceinline__ df df_add(df a, df b)
    return fast_two_sum(s.h, fadd(s.l, fadd(a.l, b.l)));
 }
 
-// a + b when |a.h| >= |b.h| is known.
-__host__ __device__ __forceinline__ df df_add_fast(df a, df b)
-{
-   const df s = fast_two_sum(a.h, b.h);
-   return fast_two_sum(s.h, fadd(s.l, fadd(a.l, b.l)));
-}
-
 __host__ __device__ __forceinline__ df df_neg(df a) { return {-a.h, -a.l}; }
-
-__host__ __device__ __forceinline__ df df_mul(df a, df b)
-{
-   const float p = fmul(a.h, b.h);
-   float e = ffma(a.h, b.h, -p);
-   e = ffma(a.h, b.l, e);
-   e = ffma(a.l, b.h, e);
-   return fast_two_sum(p, e);
-}
 
 // Product left unnormalised (p + e with |e| <= ~ulp(p)); saves the final Fast2Sum.
 __host__ __device__ __forceinline__ df df_mul_u(df a, df b)
@@ -178,14 +162,6 @@ __host__ __device__ __forceinline__ df df_mul_u(df a, df b)
    float e = ffma(a.h, b.h, -p);
    e = ffma(a.h, b.l, e);
    e = ffma(a.l, b.h, e);
-   return {p, e};
-}
-
-__host__ __device__ __forceinline__ df df_sqr_u(df a)
-{
-   const float p = fmul(a.h, a.h);
-   float e = ffma(a.h, a.h, -p);
-   e = ffma(2.0f * a.h, a.l, e);
    return {p, e};
 }
 
@@ -882,8 +858,7 @@ __host__ __device__ __forceinline__ bool collide_f64x_fast(uint64_t (&bits)[Q], 
    return true;
 }
 
-// F64X cell update with a uniform force: fast path, else the exact IEEE
-// double collision.
+// The fast path's constants from the launch parameters.
 template <int Q>
 __host__ __device__ __forceinline__ x64::Consts collide_consts(const KParams& p)
 {

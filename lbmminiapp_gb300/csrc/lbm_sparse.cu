@@ -126,10 +126,8 @@ __global__ void __launch_bounds__(kSparseThreads, sparse_min_blocks<Q>()) sparse
 // set, disjoint from every other point's.
 // Warps per block and blocks per SM: 12 warps at up to 168 registers, whose shared
 // memory fits the 164 KB carve-out (lbm_step_async.cuh says why that matters).
-template <int Q>
-constexpr int sparse_warps() { return 4; }
-template <int Q>
-constexpr int sparse_blocks() { return 3; }
+constexpr int kSparseWarps = 4;
+constexpr int kSparseBlocks = 3;
 // The D3Q27 rest population in a register, as there.
 template <int Q>
 constexpr bool sparse_rest() { return Q == 27; }
@@ -152,7 +150,7 @@ struct SparseEmit {
 };
 
 template <int Q, int KIND, int FORCE>
-__global__ void __launch_bounds__(sparse_warps<Q>() * 32, sparse_blocks<Q>()) sparse_async_kernel(
+__global__ void __launch_bounds__(kSparseWarps * 32, kSparseBlocks) sparse_async_kernel(
    const KParams p, const int32_t* __restrict__ adj, uint32_t nf, uint32_t start, uint32_t count, uint32_t ntiles,
    const double* src, double* dst)
 {
@@ -255,27 +253,26 @@ cudaError_t launch_sparse_async_form(const KParams& p, const int32_t* adj, int64
    cudaError_t e = cudaGetDevice(&dev);
    if (e != cudaSuccess) return e;
    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-   constexpr int kWarps = sparse_warps<Q>(), kBlocks = sparse_blocks<Q>();
    auto kern = sparse_async_kernel<Q, KIND, FORCE>;
-   constexpr size_t smem = (size_t)kWarps * kAsyncStages * (sparse_rest<Q>() ? Q - 1 : Q) * 32 * sizeof(unsigned long long);
+   constexpr size_t smem = (size_t)kSparseWarps * kAsyncStages * (sparse_rest<Q>() ? Q - 1 : Q) * 32 * sizeof(unsigned long long);
    int cached = grid_of_device[dev].load(std::memory_order_relaxed);
    if (cached == 0) {
       e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
-      e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, carveout_percent(kBlocks, smem));
+      e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, carveout_percent(kSparseBlocks, smem));
       if (e != cudaSuccess) return e;
       int per_sm = 0, nsm = 0;
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kWarps * 32, smem);
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSparseWarps * 32, smem);
       if (e != cudaSuccess) return e;
       e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
       if (e != cudaSuccess) return e;
-      if (per_sm < kBlocks) return cudaErrorInvalidConfiguration;
-      cached = kBlocks * nsm;   // no more than the carve-out is meant for
+      if (per_sm < kSparseBlocks) return cudaErrorInvalidConfiguration;
+      cached = kSparseBlocks * nsm;   // no more than the carve-out is meant for
       grid_of_device[dev].store(cached, std::memory_order_relaxed);
    }
    const uint32_t ntiles = (uint32_t)((count + 31) / 32);
-   const AsyncLaunch L = async_launch(ntiles, (uint32_t)cached / kBlocks, kBlocks, kWarps);
-   return launch_overlapped(kern, dim3(L.blocks), dim3(L.warps * 32), smem / kWarps * L.warps, stream, p, adj,
+   const AsyncLaunch L = async_launch(ntiles, (uint32_t)cached / kSparseBlocks, kSparseBlocks, kSparseWarps);
+   return launch_overlapped(kern, dim3(L.blocks), dim3(L.warps * 32), smem / kSparseWarps * L.warps, stream, p, adj,
                             (uint32_t)nfluid, (uint32_t)start, (uint32_t)count, ntiles, src, dst);
 }
 
