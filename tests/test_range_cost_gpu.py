@@ -1,5 +1,5 @@
 """F64X steps made by range calls against full steps, in time: the one-cell kernel of
-the ranges stays within 1.45 of the pipelined kernel (measured 1.15 to 1.3 with two
+the ranges stays within 1.45 of the pipelined kernel (measured 1.04 to 1.24 with two
 blocks per SM, from 1.5 to 2.4 with one)."""
 import pytest
 
